@@ -25,9 +25,8 @@
 //     h[end], the last-j row-max tie, z-drop, band narrowing).  The row lives
 //     in shared memory, [column][thread]: a 16-bit (int8 scores) or 32-bit
 //     (int16) H|E word and a query byte per column.  A class bound sizes only
-//     these rows; bounds that are multiples of 16 get a kernel instance with
-//     the bound as a constant.  A warp whose tasks all keep their whole query
-//     runs the plain row code, else the ring form.
+//     these rows.  A warp whose tasks all keep their whole query runs the
+//     plain row code, else the ring form.
 //   * The int32 bin runs one warp per extension for queries up to 4096
 //     (swb_ext_warp.cuh) and one thread per extension over int32 rows in
 //     global scratch above that (swb_ext_dp.cuh).
@@ -132,15 +131,14 @@ __global__ void bin_bounds_kernel(const uint32_t *__restrict__ sorted_keys, size
         for (int bb = b + 1; bb <= nbins; ++bb) bin_start[bb] = (uint32_t)n;
 }
 
-// QMAX > 0: the class bound as a constant (the multiples of 16 from 32 to
-// 256); QMAX = 0: any other bound, passed in qcap.
-template <int QMAX, int T, bool U8>
-__global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qcap_arg) {
+// qcap: the bin's class bound.  (An instance per bound, with it as a constant,
+// ran 1-4 % slower than this one: 31 instances' code for an inner loop that
+// does not use the bound.)
+template <int T, bool U8>
+__global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qcap) {
     extern __shared__ uint32_t sm[];
     // Rows: (qcap + 1) words of 2 (int8 scores) or 4 bytes (int16), then
-    // qcap + 1 query bytes; qcap is the bin's class bound (the rows' only use
-    // of it).
-    const int qcap = QMAX > 0 ? QMAX : qcap_arg;
+    // qcap + 1 query bytes.
     uint16_t *he16 = reinterpret_cast<uint16_t *>(sm) + threadIdx.x;
     uint32_t *he32 = sm + threadIdx.x;
     uint8_t *qc = reinterpret_cast<uint8_t *>(sm) + (size_t)(qcap + 1) * T * (U8 ? 2 : 4) + threadIdx.x;
@@ -339,19 +337,7 @@ const char *bin_name(bool u8, int qcap) {
 
 using FastKernel = void (*)(ExtArgs, int, int);
 
-template <bool U8, int... Q>
-FastKernel fast_kernel_for(int qcap, std::integer_sequence<int, Q...>) {
-    FastKernel k = ext_fast_kernel<0, kFastT, U8>;
-    ((qcap == 32 + 16 * Q ? (void)(k = ext_fast_kernel<32 + 16 * Q, kFastT, U8>) : (void)0), ...);
-    return k;
-}
-
-// The kernel instance for a class bound: the constant-bound one for the
-// multiples of 16 from 32 to 256, else the runtime-bound one.
-FastKernel fast_kernel(bool u8, int qcap) {
-    return u8 ? fast_kernel_for<true>(qcap, std::make_integer_sequence<int, 15>{})
-              : fast_kernel_for<false>(qcap, std::make_integer_sequence<int, 15>{});
-}
+FastKernel fast_kernel(bool u8) { return u8 ? ext_fast_kernel<kFastT, true> : ext_fast_kernel<kFastT, false>; }
 
 // Resident one-warp blocks per SM of the shared-memory kernel for a class bound.
 int fast_occupancy(bool u8, int qcap) {
@@ -364,7 +350,7 @@ int fast_occupancy(bool u8, int qcap) {
     int &occ = cache[u8 ? 1 : 0][qcap];
     if (occ < 0) {
         int o = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8, qcap), kFastT, fast_smem_bytes(qcap, u8)) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8), kFastT, fast_smem_bytes(qcap, u8)) !=
             cudaSuccess)
             return -1;
         occ = o < 1 ? 1 : o;
@@ -379,7 +365,7 @@ int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, int qcap, size
     if (grid == 0) return SWB_OK;
     const size_t smem = fast_smem_bytes(qcap, u8);
     ProfScope ps(ctx, s, ctx->prof_on ? bin_name(u8, qcap) : nullptr, kCntExtBin0 + bin);
-    fast_kernel(u8, qcap)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
+    fast_kernel(u8)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
     return SWB_OK;
