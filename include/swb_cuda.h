@@ -262,9 +262,11 @@ int swb_ext_batch_plain_device(swb_ctx *ctx, const swb_scoring *sc,
                                size_t n_tasks, swb_ext_result *d_out, void *stream);
 
 /* Length classes of the extension bins: ascending bounds on the row length
- * a task keeps, min(qlen, 2w + 2) with w the band after the reference's
- * clamp (BandedSWScalar.swift:52-62) -- a band narrower than the query is
- * kept as a ring of its columns -- as 1..15 values within [8, 256]; each
+ * a task keeps -- the query columns from the first row it computes on (rows
+ * before the first mismatch may be left out), or for a query longer than the
+ * last bound min(qlen, 2w + 2) with w the band after the reference's clamp
+ * (BandedSWScalar.swift:52-62), a band narrower than the query being kept as
+ * a ring of its columns -- as 1..15 values within [8, 256]; each
  * class has an int8-row and an int16-row bin (two target rows per pass, one
  * task per thread), and rows above the last bound, or scores beyond int16,
  * run one warp per extension.  Defaults: 32 48 64 80 96 112 128 160 192 256.
@@ -541,7 +543,11 @@ int swb_local_align(swb_ctx *ctx, const uint8_t *query, int32_t qlen,
 /* Per-kernel accounting.  With profiling on, every kernel launch is
  * bracketed by CUDA events on its stream; swb_profile_read synchronises the
  * context's streams and returns, per kernel name, the launches, summed
- * device time and DP cells since the last swb_profile_reset. */
+ * device time and DP cells since the last swb_profile_reset.  The extension
+ * kernels then compute every row the reference computes, so that the cells are
+ * its count; without profiling they leave out rows that cannot change a
+ * result (swb_ext_batch, whose cells swb_last_batch_stats reports, never
+ * does), so a pass takes longer under profiling. */
 typedef struct swb_kernel_stat {
     char     name[40];
     uint32_t launches;
@@ -561,7 +567,8 @@ int swb_int16x2_alu_peak(swb_ctx *ctx, double *lane_ops_per_s);
 /* Kernel launches issued by this context so far (for launch accounting). */
 uint64_t swb_kernel_launches(const swb_ctx *ctx);
 /* Device time (ms, CUDA events on the context's stream) of the last
- * synchronous batch call's kernels, and DP cells it updated. */
+ * synchronous batch call's kernels, and the DP cells it updated (for
+ * swb_ext_batch those of every row the reference computes). */
 int swb_last_batch_stats(const swb_ctx *ctx, double *kernel_ms, uint64_t *cells);
 
 #ifdef __cplusplus

@@ -6,10 +6,11 @@
 //     int8 rows when the score bound h0 + qlen*maxScore is at most 255,
 //     int16 rows when it is at most 32000, each in the context's length
 //     classes (ExtBins: up to 15 bounds, defaults 32..256, chosen by
-//     swb_tune_ext_bins) of the columns the task keeps: min(qlen, 2w + 2)
-//     (ext_row_len: a band narrower than the query is kept as a ring) in
-//     passes of kRingAllTasks tasks and up, else its query length unless
-//     the query is longer than the last bound;
+//     swb_tune_ext_bins) of the columns the task keeps: those of its query
+//     from its first row computed on (rows before the first mismatch are left
+//     out, swb_ext_skip.cuh), or for a query longer than the last bound
+//     min(qlen, 2w + 2) (ext_row_len: a band narrower than the query is kept
+//     as a ring);
 //     everything else (rows above the last bound, larger scores, gap costs
 //     beyond a 16-bit lane) goes to the int32 bin.
 //     The bounds are static, so no row ever saturates and nothing is re-run.
@@ -58,24 +59,21 @@ constexpr int kFastT = 32;                // threads per block in the shared-mem
 // byte 256, the bins' claim counters from byte 320.
 constexpr size_t kMiscBytes = 512;
 constexpr int kBigT = 64;
+// Rows past the query's length that a task is taken to run when it may stop
+// early (sort key only).
+constexpr int kTailRows = 4;
 
 // True when every H/E of the task fits one byte: H <= h0 + qlen*maxMat.
 __device__ __forceinline__ bool fits8(int qlen, int h0, int max_mat) {
     return h0 >= 0 && (long long)h0 + (long long)qlen * (max_mat > 0 ? max_mat : 0) <= 255;
 }
 
-// Columns the two-row code keeps for a task (less one): the query length,
-// or for queries longer than `ring_above` the band's ring, ext_row_len.
-// A pass of fewer than kRingAllTasks tasks sets ring_above to the last
-// length class, so only queries beyond the classes take rings: binning by
-// ring length mixes tasks of very different row counts in a bin, and a
-// small pass ends with its slowest bin -- a serving wave of 131k
-// config-2-like tasks ran a third slower that way (100M -> 67M ext/s).  A
-// larger pass (0: every task whose band is narrower than its query) is
-// bound by throughput and gains from the occupancy (20M config-2 tasks:
-// 146.4 -> 141.3 ms).  Tasks beyond the classes take the int32 bin either
-// way, since a ring is never longer than the query.
-constexpr size_t kRingAllTasks = size_t(1) << 22;
+// Columns the two-row code keeps for a task (less one): the query length, or
+// for queries longer than `ring_above`, the last length class, the band's
+// ring, ext_row_len (which keeps narrow bands out of the int32 bin).  Rings for
+// every band narrower than its query gained from the occupancy when all rows
+// were computed (20M uneven tasks 146.4 -> 143.8 ms) but not since rows are left
+// out, which rings do not do (5M uneven tasks: 31.2 ms against 32.1).
 __device__ __host__ __forceinline__ int task_row_len(const swb_ext_task &t, const DevScoring &sc, int ring_above) {
     return t.qlen > ring_above ? ext_row_len(t.qlen, ext_band_w(t.qlen, t.w, t.end_bonus, sc)) : t.qlen;
 }
@@ -83,11 +81,12 @@ __device__ __host__ __forceinline__ int task_row_len(const swb_ext_task &t, cons
 // pair_ok: the gap costs fit a 16-bit lane (the two-row kernels of both row
 // widths); otherwise every task takes the int32 bin.  Columns run in 16-bit
 // lanes, so queries above kMaxLen take it too (and are refused there).
+// len: the columns the task keeps (task_row_len, less those before its first
+// row computed).
 __device__ __forceinline__ int ext_bin(const swb_ext_task &t, const DevScoring &sc, bool pair_ok, uint32_t warp_cells,
-                                       const ExtBins &bins, int ring_above) {
+                                       const ExtBins &bins, int len) {
     if (t.qlen <= 0 || t.tlen <= 0) return 0;
     const int big = 2 * bins.n;
-    const int len = task_row_len(t, sc, ring_above);
     if (!pair_ok || len > bins.q[bins.n - 1] || t.qlen > kMaxLen || !fits16(t.qlen, t.h0, sc.max_mat)) return big;
     if (warp_cells && (unsigned long long)t.qlen * (unsigned long long)t.tlen > warp_cells) return big;
     int b = 0;
@@ -95,22 +94,37 @@ __device__ __forceinline__ int ext_bin(const swb_ext_task &t, const DevScoring &
     return fits8(t.qlen, t.h0, sc.max_mat) ? b : bins.n + b;
 }
 
-// Sort key: bin in bits 27-31, then target length (the rows a task runs) and
-// row length, longest first: within a bin the tasks with the most rows start
-// first, so a band narrower than its query (a short ring row over many
-// target rows) does not start last and hold the bin up.
+// Sort key: bin in bits 27-31, then the band's half-width in steps of 16
+// columns (4 bits), the rows the task runs (12) and its row length (11), each
+// largest first: the lanes of a warp run similar numbers of rows of similar
+// width, and within a bin the tasks with the most work start first and overlap
+// the rest instead of finishing the bin alone.  The rows are those after the
+// ones left out at the start (skip[i], ext_skip_rows), up to the target's end,
+// or with all = 0 about the query's length, where most tasks stop.
 __global__ void ext_keys_kernel(const swb_ext_task *__restrict__ tasks, size_t n, DevScoring sc, int pair_ok,
-                                uint32_t warp_cells, ExtBins bins, int ring_above, uint32_t *__restrict__ keys,
-                                uint32_t *__restrict__ idx, int *__restrict__ big_max_q) {
+                                uint32_t warp_cells, ExtBins bins, int ring_above, int all, int skip_rows,
+                                const uint8_t *__restrict__ bases, const uint8_t *__restrict__ pac,
+                                uint32_t *__restrict__ keys, uint32_t *__restrict__ idx, uint16_t *__restrict__ skip,
+                                int *__restrict__ big_max_q) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const swb_ext_task t = tasks[i];
-    const int b = ext_bin(t, sc, pair_ok != 0, warp_cells, bins, ring_above);
-    const uint32_t q = (uint32_t)min(max(b < 2 * bins.n ? task_row_len(t, sc, ring_above) : t.qlen, 0), 4095);
-    const uint32_t tl = (uint32_t)min(max(t.tlen, 0), 32767);
-    // Within a bin the longest tasks come first: they are claimed first, so
-    // they overlap the rest instead of finishing the bin alone.
-    keys[i] = ((uint32_t)b << 27) | ((32767u - tl) << 12) | (4095u - q);
+    int len = task_row_len(t, sc, ring_above), s = 0;
+    int b = ext_bin(t, sc, pair_ok != 0, warp_cells, bins, len);
+    const bool pair = b < 2 * bins.n && t.qlen > 0 && t.tlen > 0;
+    if (pair && skip_rows && len == t.qlen) {
+        s = ext_skip_rows(t, sc, bases, pac);
+        if (s > 0) {   // the columns left: maybe a smaller class
+            len -= ext_start_col(sc, ext_band_w(t.qlen, t.w, t.end_bonus, sc), t.h0, s);
+            b = ext_bin(t, sc, true, 0, bins, len);
+        }
+    }
+    skip[i] = (uint16_t)s;
+    const uint32_t q = (uint32_t)min(max(pair ? len : t.qlen, 0), 2047);
+    const int rows = (pair && !all ? min(t.tlen, t.qlen + kTailRows) : t.tlen) - s;
+    const uint32_t wide = (uint32_t)min(max(min(t.w, t.qlen), 0) >> 4, 15);
+    keys[i] = ((uint32_t)b << 27) | ((15u - wide) << 23) | ((4095u - (uint32_t)min(max(rows, 0), 4095)) << 11) |
+              (2047u - q);
     idx[i] = (uint32_t)i;
     if (b == 2 * bins.n) atomicMax(big_max_q, t.qlen);
 }
@@ -134,7 +148,7 @@ __global__ void bin_bounds_kernel(const uint32_t *__restrict__ sorted_keys, size
 // qcap: the bin's class bound.  (An instance per bound, with it as a constant,
 // ran 1-4 % slower than this one: 31 instances' code for an inner loop that
 // does not use the bound.)
-template <int T, bool U8>
+template <int T, bool U8, bool ALL>
 __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qcap) {
     extern __shared__ uint32_t sm[];
     // Rows: (qcap + 1) words of 2 (int8 scores) or 4 bytes (int16), then
@@ -160,28 +174,24 @@ __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qca
             ti = a.order[pos];
             tk = a.tasks[ti];
         }
-        // The ring form only for warps that hold a task whose band is
-        // narrower than its query.
-        const bool ring = __any_sync(0xFFFFFFFFu, pos < hi && task_row_len(tk, a.sc, a.ring_above) < tk.qlen);
+        // The ring form only for warps that hold a ring task, and there for all
+        // lanes whose rows hold the whole query too.
+        const bool rings = __any_sync(0xFFFFFFFFu, pos < hi && task_row_len(tk, a.sc, a.ring_above) < tk.qlen);
         if (pos < hi) {
             swb_ext_result r;
             const bool sym = a.sc.o_del + a.sc.e_del == a.sc.o_ins + a.sc.e_ins;
-            if (ring) {
-                if constexpr (U8) {
-                    if (sym) ext_pair_one<T, true, false, true>(a, tk, he16, qc, r, cells);
-                    else ext_pair_one<T, false, false, true>(a, tk, he16, qc, r, cells);
-                } else {
-                    if (sym) ext_pair_one<T, true, true, true>(a, tk, he32, qc, r, cells);
-                    else ext_pair_one<T, false, true, true>(a, tk, he32, qc, r, cells);
-                }
+            const int skip = a.skip[ti];
+            auto run = [&](auto symc, auto ringc) {
+                constexpr bool kSym = decltype(symc)::value, kRing = decltype(ringc)::value;
+                if constexpr (U8) ext_pair_one<T, kSym, false, kRing, ALL>(a, tk, skip, he16, qc, r, cells);
+                else ext_pair_one<T, kSym, true, kRing, ALL>(a, tk, skip, he32, qc, r, cells);
+            };
+            if (rings && skip == 0) {
+                if (sym) run(std::true_type{}, std::true_type{});
+                else run(std::false_type{}, std::true_type{});
             } else {
-                if constexpr (U8) {
-                    if (sym) ext_pair_one<T, true, false, false>(a, tk, he16, qc, r, cells);
-                    else ext_pair_one<T, false, false, false>(a, tk, he16, qc, r, cells);
-                } else {
-                    if (sym) ext_pair_one<T, true, true, false>(a, tk, he32, qc, r, cells);
-                    else ext_pair_one<T, false, true, false>(a, tk, he32, qc, r, cells);
-                }
+                if (sym) run(std::true_type{}, std::false_type{});
+                else run(std::false_type{}, std::false_type{});
             }
             a.out[ti] = r;
         }
@@ -307,12 +317,13 @@ __global__ void __launch_bounds__(T) ext_plain_kernel(ExtArgs a, size_t n, int q
         if (plain_pair_task(tk, a.sc.max_mat, pair_ok != 0)) {
             swb_ext_result r;
             const bool sym = a.sc.o_del + a.sc.e_del == a.sc.o_ins + a.sc.e_ins;
+            // (No rows left out: unsorted, a warp's tasks rarely all have some.)
             if constexpr (U8) {
-                if (sym) ext_pair_one<T, true, false, false>(a, tk, he16, qc, r, cells);
-                else ext_pair_one<T, false, false, false>(a, tk, he16, qc, r, cells);
+                if (sym) ext_pair_one<T, true, false, false, true>(a, tk, 0, he16, qc, r, cells);
+                else ext_pair_one<T, false, false, false, true>(a, tk, 0, he16, qc, r, cells);
             } else {
-                if (sym) ext_pair_one<T, true, true, false>(a, tk, he32, qc, r, cells);
-                else ext_pair_one<T, false, true, false>(a, tk, he32, qc, r, cells);
+                if (sym) ext_pair_one<T, true, true, false, true>(a, tk, 0, he32, qc, r, cells);
+                else ext_pair_one<T, false, true, false, true>(a, tk, 0, he32, qc, r, cells);
             }
             a.out[pos] = r;
         }
@@ -337,20 +348,23 @@ const char *bin_name(bool u8, int qcap) {
 
 using FastKernel = void (*)(ExtArgs, int, int);
 
-FastKernel fast_kernel(bool u8) { return u8 ? ext_fast_kernel<kFastT, true> : ext_fast_kernel<kFastT, false>; }
+FastKernel fast_kernel(bool u8, bool all) {
+    if (all) return u8 ? ext_fast_kernel<kFastT, true, true> : ext_fast_kernel<kFastT, false, true>;
+    return u8 ? ext_fast_kernel<kFastT, true, false> : ext_fast_kernel<kFastT, false, false>;
+}
 
 // Resident one-warp blocks per SM of the shared-memory kernel for a class bound.
-int fast_occupancy(bool u8, int qcap) {
-    static int cache[2][kExtSmemMaxQ + 1];
+int fast_occupancy(bool u8, bool all, int qcap) {
+    static int cache[4][kExtSmemMaxQ + 1];
     static std::once_flag once;
     std::call_once(once, [] {
         for (auto &row : cache)
             for (int &v : row) v = -1;
     });
-    int &occ = cache[u8 ? 1 : 0][qcap];
+    int &occ = cache[(u8 ? 1 : 0) + (all ? 2 : 0)][qcap];
     if (occ < 0) {
         int o = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8), kFastT, fast_smem_bytes(qcap, u8)) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8, all), kFastT, fast_smem_bytes(qcap, u8)) !=
             cudaSuccess)
             return -1;
         occ = o < 1 ? 1 : o;
@@ -358,14 +372,14 @@ int fast_occupancy(bool u8, int qcap) {
     return occ;
 }
 
-int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, int qcap, size_t n, cudaStream_t s) {
-    const int occ = fast_occupancy(u8, qcap);
+int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, cudaStream_t s) {
+    const int occ = fast_occupancy(u8, all, qcap);
     if (occ < 0) return check_cuda(cudaGetLastError(), "occupancy query");
     const size_t grid = std::min<size_t>((n + kFastT - 1) / kFastT, (size_t)ctx->sm_count * occ);
     if (grid == 0) return SWB_OK;
     const size_t smem = fast_smem_bytes(qcap, u8);
     ProfScope ps(ctx, s, ctx->prof_on ? bin_name(u8, qcap) : nullptr, kCntExtBin0 + bin);
-    fast_kernel(u8)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
+    fast_kernel(u8, all)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
     return SWB_OK;
@@ -380,7 +394,7 @@ int ext_reserve(swb_ctx *ctx, size_t cap) {
     SWB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr,
                                              (uint32_t *)nullptr, (uint32_t *)nullptr, (int)cap, 0, 32, ctx->stream));
     if ((rc = ensure_dev(ctx, ctx->d_keys, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_keys2, cap * 4)) ||
-        (rc = ensure_dev(ctx, ctx->d_idx, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, 2 * cap * 4)) ||
+        (rc = ensure_dev(ctx, ctx->d_idx, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, 2 * cap * 6)) ||
         (rc = ensure_dev(ctx, ctx->d_misc, 2 * kMiscBytes)) || (rc = ensure_dev(ctx, ctx->d_sort_tmp, tmp_bytes)))
         return rc;
     return SWB_OK;
@@ -389,7 +403,7 @@ int ext_reserve(swb_ctx *ctx, size_t cap) {
 int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
                const swb_ext_task *d_tasks, size_t n, swb_ext_result *d_out,
                unsigned long long *d_cells, cudaStream_t s, int max_q_hint, uint32_t warp_cells,
-               const ExtPipe *pipe) {
+               const ExtPipe *pipe, bool all_rows) {
     if (n == 0) return SWB_OK;
     if (n > 0x7FFFFFF0ull) return set_error(SWB_ERR_TOO_LARGE, "more than 2^31-16 tasks in one batch");
     if (pipe && n > pipe->cap) return set_error(SWB_ERR_INVALID_ARG, "pass larger than its scratch set");
@@ -400,16 +414,28 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     const size_t set = pipe ? pipe->cap : n;
     const int slot = pipe ? pipe->slot : 0;
     if ((rc = ensure_dev(ctx, ctx->d_keys, n * 4)) || (rc = ensure_dev(ctx, ctx->d_keys2, n * 4)) ||
-        (rc = ensure_dev(ctx, ctx->d_idx, n * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, (slot + 1) * set * 4)) ||
+        (rc = ensure_dev(ctx, ctx->d_idx, n * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, (slot + 1) * set * 6)) ||
         (rc = ensure_dev(ctx, ctx->d_misc, (slot + 1) * kMiscBytes)))
         return rc;
     // The context's length classes at the time of the call: the keys and the
     // launches below use the same copy.
     const ExtBins bins = ctx->ext_bins;
-    const int ring_above = n >= kRingAllTasks ? 0 : bins.q[bins.n - 1];
+    // Rows that cannot change a result are computed only where the reference's
+    // cell count is reported: by the host batch entry and under profiling.
+    const bool all = all_rows || ctx->prof_on;
+    const int ring_above = bins.q[bins.n - 1];
+    // The rows before the first mismatch are left out in passes of more tasks
+    // than the GPU holds lanes of these kernels (about 20 one-warp blocks per
+    // SM).  A smaller pass lasts as long as its longest task, and lanes that
+    // start at different rows take longer over each (uneven tasks, rows left out
+    // / kept: 8k 1455 / 1242 us, 64k 1436 / 1330, 256k 2169 / 2310, 1M 6679 / 7731;
+    // 150 bp reads: 16k 532 / 533, 64k 684 / 710, 1M 2232 / 2998).
+    const int skip_rows = n > (size_t)ctx->sm_count * 20 * kFastT;
     const int nbins = 2 * bins.n + 1, big = 2 * bins.n;
     uint32_t *keys = (uint32_t *)ctx->d_keys.p, *keys2 = (uint32_t *)ctx->d_keys2.p;
     uint32_t *idx = (uint32_t *)ctx->d_idx.p, *idx2 = (uint32_t *)ctx->d_idx2.p + (size_t)slot * set;
+    // The rows each task leaves out, behind the sets' orders.
+    uint16_t *skip = (uint16_t *)((uint32_t *)ctx->d_idx2.p + (pipe ? 2 : 1) * set) + (size_t)slot * set;
     char *misc = (char *)ctx->d_misc.p + slot * kMiscBytes;
     uint32_t *bin_start = (uint32_t *)misc;                   // nbins + 1 words
     int *big_max_q = (int *)(misc + 256);
@@ -421,7 +447,8 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         // Two target rows per pass on 16-bit lanes: the gap costs must fit a lane.
         const int pair_ok = sc.o_del + sc.e_del <= 32767 && sc.o_ins + sc.e_ins <= 32767;
         ext_keys_kernel<<<(unsigned)((n + tb - 1) / tb), tb, 0, s>>>(d_tasks, n, sc, pair_ok, warp_cells, bins,
-                                                                       ring_above, keys, idx, big_max_q);
+                                                                       ring_above, all, skip_rows, d_bases, ctx->d_pac,
+                                                                       keys, idx, skip, big_max_q);
     }
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
@@ -468,7 +495,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
 
     // Fork: every bin runs on its own stream after the sort, then joins back
     // (into the pipeline's join stream for pipelined passes).
-    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, d_cells, claim, ring_above};
+    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, d_cells, claim, ring_above, skip};
     const cudaStream_t js = pipe ? pipe->join : s;
     ProfScope pass(ctx, s, pipe ? nullptr : "ext_pass", -1);   // fork to join, on the launching stream
     SWB_CUDA(cudaEventRecord(ctx->fork_ev, s));
@@ -476,7 +503,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         cudaStream_t sb = ctx->side[b];
         SWB_CUDA(cudaStreamWaitEvent(sb, ctx->fork_ev, 0));
         if (b < big) {
-            if ((rc = launch_fast(ctx, a, b, b < bins.n, bins.q[b % bins.n], n, sb))) return rc;
+            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], n, sb))) return rc;
         } else if (max_q > 0) {
             ProfScope ps(ctx, sb, "ext_big_i32", kCntExtBin0 + big);
             ext_warp_kernel<<<(unsigned)wblocks, wwarps * 32, wwarps * wstride, sb>>>(a, big, wq);

@@ -50,12 +50,22 @@
 // when M > 0 and 0 when M = 0: M*128 for byte scores, a 0/1 lane mask times
 // 0x7FFF for 16-bit ones.  The row max (last column on ties) is a u16x2 key
 // H*256 + j for byte scores and one s32 key (H << 16) + j per row otherwise.
+// Rows left out at the start: those before the task's first mismatch
+// (swb_ext_skip.cuh).
+// Rows left out at the end (ALL = false): once gScore > 0 and no cell can
+// reach either best, even matching every query base left -- H + a*(bases
+// left) below gScore and not above maxScore, for every nonzero word -- the
+// rows left change nothing (a path only loses by gaps, a zero cell starts
+// none, z-drop and an empty row only stop earlier).  ALL = true computes them,
+// for callers that report the reference's cell count; the skipped first rows'
+// cells are counted from the band either way.
 #pragma once
 
 #include <type_traits>
 
 #include "swb_device.cuh"
 #include "swb_ext_dp.cuh"
+#include "swb_ext_skip.cuh"
 
 namespace swb {
 namespace {
@@ -147,9 +157,10 @@ struct RowTrack {
     }
 };
 
-template <int T, bool SYM, bool W16, bool RING>
-__device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_task &tk, RowWord<W16> *__restrict__ he,
-                                             uint8_t *__restrict__ qc, swb_ext_result &res,
+// skip: ext_skip_rows of the task, or 0 (a ring takes 0).
+template <int T, bool SYM, bool W16, bool RING, bool ALL>
+__device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_task &tk, int skip,
+                                             RowWord<W16> *he, uint8_t *qc, swb_ext_result &res,
                                              unsigned long long &cells) {
     using Word = RowWord<W16>;
     constexpr uint32_t kLoMask = W16 ? 0xFFFFu : 0xFFu;      // one score field of a word
@@ -178,24 +189,48 @@ __device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_tas
             return r >= P ? r - P : r;
         }
     };
-    // Query profile and the first row from h0 (:44-50, :65-77); with a ring,
-    // the columns that fit it (the rest enter with the band, below).
-    {
+    // First-row value of column c > 0 (:65-77).
+    auto ramp = [&](int c) -> int {
+        const long long v = h0 > oIns + eIns ? (long long)h0 - oIns - (long long)eIns * c : 0;
+        return v > 0 ? (int)v : 0;
+    };
+    RowTrack tr{h0, -1, -1, -1, -1, 0};
+    int beg = 0, end = qlen;
+    const int i0 = RING ? 0 : skip;
+    // Query profile and the words before the first row computed.
+    if (RING || i0 == 0) {
+        // The first row from h0 (:44-50, :65-77); with a ring, the columns
+        // that fit it (the rest enter with the band, below).
         int hv = h0;
-        bool ramp = h0 > oIns + eIns;
+        bool down = h0 > oIns + eIns;
         for (int j = 0; j < P; ++j) {
             int hj = 0;
             if (j == 0) {
                 hj = h0;
             } else if (j == 1) {
-                if (ramp) hj = hv = h0 - oIns - eIns;
-            } else if (ramp && hv > eIns) {
+                if (down) hj = hv = h0 - oIns - eIns;
+            } else if (down && hv > eIns) {
                 hj = hv -= eIns;
             } else {
-                ramp = false;
+                down = false;
             }
             if (j < qlen) qc[j * T] = (uint8_t)span_base(a.bases, a.pac, tk.q_off, j, qlen, tk.flags, false);
             he[j * T] = (Word)hj;
+        }
+    } else {
+        const ExtStart st = ext_start<ALL>(sc, qlen, w, h0, i0, cells);
+        beg = st.beg;
+        end = st.end;
+        tr = RowTrack{st.dLast, i0 - 1, i0 - 1, st.gScore, st.gTle, 0};
+        // No column before the first one is touched again: the rows start there.
+        const int off = ext_start_col(sc, w, h0, i0);
+        he -= off * T;
+        qc -= off * T;
+        for (int j = off; j <= qlen; ++j) {
+            int hj, ej;
+            st.word(sc, h0, j, hj, ej);
+            if (j < qlen) qc[j * T] = (uint8_t)span_base(a.bases, a.pac, tk.q_off, j, qlen, tk.flags, false);
+            he[j * T] = (Word)((uint32_t)hj | ((uint32_t)ej << (W16 ? 16 : 8)));
         }
     }
     const bool tref = (tk.flags & SWB_T_FROM_REF) != 0;
@@ -212,14 +247,7 @@ __device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_tas
         return (uint32_t)imax(h0 - (oDel + eDel * (row + 1)), 0);
     };
 
-    // Ring: the first-row value of a column entering the ring (:65-77).
-    auto ramp = [&](int c) -> int {
-        const long long v = h0 > oIns + eIns ? (long long)h0 - oIns - (long long)eIns * c : 0;
-        return v > 0 ? (int)v : 0;
-    };
-    RowTrack tr{h0, -1, -1, -1, -1, 0};
-    int beg = 0, end = qlen;
-    int i = 0;
+    int i = i0;
     while (i < tlen) {
         if constexpr (RING) {
             // Slide the ring's base with the band, then bring in the columns
@@ -379,6 +407,27 @@ __device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_tas
         const int ne = imin((int)(lj1 & 0xFFFFu), e1 - 1) + 1;
         end = imin(ne + 2, qlen);
         i += 2;
+        if constexpr (!ALL) {
+            // No cell can reach a best any more (see the header)?  From the
+            // diagonal's last row on; the scan meets a cell that can, near
+            // the alignment's column, after few words.
+            // Words past `end` are zero, or past column w + 1 the first row's,
+            // which a band that grows again may still read.
+            const int A = imax(sc.a, 0);
+            const int limit = imin(tr.gScore, tr.maxScore + 1);
+            const int stale = w + 2 <= qlen ? ramp(w + 2) : 0;
+            if (i >= qlen && tr.gScore > 0 && (stale == 0 || stale + A * (qlen - w - 2) < limit)) {
+                int j = imin(end, qlen - 1);
+                if constexpr (RING) j = imin(j, i + w);                        // the columns that entered
+                for (; j >= beg; --j) {
+                    const uint32_t wd = he[sl(j) * T];
+                    const int hv = (int)(wd & kLoMask), ev = (int)(W16 ? wd >> 16 : wd >> 8);
+                    const int left = A * (qlen - j);
+                    if (wd != 0u && imax(hv > 0 ? hv + left : 0, ev > 0 ? ev + left - A : 0) >= limit) break;
+                }
+                if (j < beg) break;
+            }
+        }
     }
     res = swb_ext_result{tr.maxScore, tr.maxJ + 1, tr.maxI + 1, tr.gTle + 1, tr.gScore, tr.maxOff};   // :183-190
 }

@@ -206,6 +206,8 @@ int ensure_host(swb_ctx *ctx, HostBuf &b, size_t bytes);
 // Extension (kernel 1).  d_tasks/d_out are device arrays of n tasks/results.
 // warp_cells > 0: tasks with more DP cells (qlen * tlen) run one warp per
 // extension (latency), otherwise their length bin's thread-per-task kernel.
+// all_rows: compute every row the reference does, so that `cells` receives the
+// reference's count; else rows that cannot change a result are left out.
 // Pipelined passes: two scratch sets let pass k+1 sort and start its bins
 // while pass k's bins finish.  The caller sizes the scratch with
 // ext_reserve(cap) first and makes `stream` wait for pass k-2 to finish
@@ -219,7 +221,7 @@ int ext_reserve(swb_ctx *ctx, size_t cap);
 int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
                const swb_ext_task *d_tasks, size_t n, swb_ext_result *d_out,
                unsigned long long *d_cells, cudaStream_t stream, int max_q_hint,
-               uint32_t warp_cells = 0, const ExtPipe *pipe = nullptr);
+               uint32_t warp_cells = 0, const ExtPipe *pipe = nullptr, bool all_rows = false);
 
 // The plain one-launch-per-batch comparator of the extension pass (the same
 // two-row kernel over the batch in input order; no sort, bins or claiming).

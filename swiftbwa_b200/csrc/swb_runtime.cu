@@ -624,7 +624,7 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
         // the GPU, the sort and the per-bin launches cost more than they save.
         rc = n_tasks <= kExtPlainMaxTasks
                  ? launch_ext_plain(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream)
-                 : launch_ext(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, big_q, 0, &pipe);
+                 : launch_ext(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, big_q, 0, &pipe, true);
         if (rc) {
             cudaStreamSynchronize(ctx->d2h);
             cudaStreamSynchronize(ctx->stream);
