@@ -228,6 +228,48 @@ __global__ void __launch_bounds__(256) ext_warp_kernel(ExtArgs a, int bin, int q
     add_cells(a.cells + kCntExtBin0 + bin, cells);
 }
 
+// Small batches (launch_ext_warps): one warp per extension, in input order;
+// queries of at most 32*KC - 1 bases (longer ones are the next kernel's).
+template <int KC>
+__global__ void __launch_bounds__(128) ext_warps_kernel(ExtArgs a, uint32_t n) {
+    unsigned long long cells = 0;
+    for (uint32_t k = blockIdx.x * 4 + (threadIdx.x >> 5); k < n; k += gridDim.x * 4) {
+        const swb_ext_task tk = a.tasks[k];
+        if (tk.qlen >= 32 * KC) continue;
+        swb_ext_result r;
+        ext_warp_regs<KC>(a, tk, r, cells);
+        if ((threadIdx.x & 31) == 0) a.out[k] = r;
+    }
+    add_cells(a.cells + kCntExtBin0, cells);
+}
+
+// The longer queries of a small batch, rows in shared memory as in the int32 bin.
+__global__ void __launch_bounds__(256) ext_warps_long_kernel(ExtArgs a, uint32_t n, int qmin, int qcap) {
+    extern __shared__ __align__(16) uint8_t wsm[];
+    const int warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const size_t stride = ((size_t)(qcap + 1) * 8 + (size_t)qcap + 15) & ~(size_t)15;
+    int *h = reinterpret_cast<int *>(wsm + warp * stride);
+    int *e = h + (qcap + 1);
+    uint8_t *qc = reinterpret_cast<uint8_t *>(e + (qcap + 1));
+    unsigned long long cells = 0;
+    for (uint32_t k = blockIdx.x * warps + warp; k < n; k += gridDim.x * warps) {
+        const swb_ext_task tk = a.tasks[k];
+        if (tk.qlen < qmin || tk.qlen > qcap) continue;
+        swb_ext_result r;
+        ext_warp_one(a, tk, h, e, qc, r, cells);
+        if ((threadIdx.x & 31) == 0) a.out[k] = r;
+        __syncwarp();
+    }
+    add_cells(a.cells + kCntExtBin0 + 1, cells);
+}
+
+// *out = the batch's longest query (0 at least).
+__global__ void max_qlen_kernel(const swb_ext_task *__restrict__ tasks, uint32_t n, int *__restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const unsigned q = __reduce_max_sync(0xFFFFFFFFu, i < n ? (unsigned)max(tasks[i].qlen, 0) : 0u);
+    if ((threadIdx.x & 31) == 0) atomicMax(out, (int)q);
+}
+
 // Queries above kWarpMaxQ: one thread per extension over int32 rows in
 // global scratch (tasks with qlen <= skip_le belong to the warp kernel).
 __global__ void __launch_bounds__(kBigT) ext_global_kernel(ExtArgs a, int bin, int *h, int *e, uint8_t *q,
@@ -400,14 +442,57 @@ int ext_reserve(swb_ctx *ctx, size_t cap) {
     return SWB_OK;
 }
 
+// Small batches: one warp per extension, one launch (two with queries above
+// kExtWarpsMaxQ), nothing read back.  max_q, the longest query, is at most
+// kWarpMaxQ.
+int launch_ext_warps(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases, const swb_ext_task *d_tasks, size_t n,
+                     swb_ext_result *d_out, unsigned long long *d_cells, cudaStream_t s, int max_q) {
+    if (n == 0) return SWB_OK;
+    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, nullptr, nullptr, d_cells};
+    const unsigned grid = (unsigned)std::min<size_t>((n + 3) / 4, (size_t)ctx->sm_count * 64);
+    {
+        ProfScope ps(ctx, s, "ext_warps", kCntExtBin0);
+        if (max_q < 32 * 4) ext_warps_kernel<4><<<grid, 128, 0, s>>>(a, (uint32_t)n);
+        else ext_warps_kernel<8><<<grid, 128, 0, s>>>(a, (uint32_t)n);
+        ctx->launches++;
+        SWB_CUDA(cudaGetLastError());
+    }
+    if (max_q > kExtWarpsMaxQ) {
+        const size_t stride = ((size_t)(max_q + 1) * 8 + (size_t)max_q + 15) & ~(size_t)15;
+        const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / stride));
+        SWB_CUDA(cudaFuncSetAttribute(ext_warps_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(warps * stride)));
+        ProfScope ps(ctx, s, "ext_warps_long", kCntExtBin0 + 1);
+        ext_warps_long_kernel<<<(unsigned)std::min<size_t>((n + warps - 1) / warps, (size_t)ctx->sm_count * 16), warps * 32,
+                                warps * stride, s>>>(a, (uint32_t)n, kExtWarpsMaxQ + 1, max_q);
+        ctx->launches++;
+        SWB_CUDA(cudaGetLastError());
+    }
+    return SWB_OK;
+}
+
 int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
                const swb_ext_task *d_tasks, size_t n, swb_ext_result *d_out,
                unsigned long long *d_cells, cudaStream_t s, int max_q_hint, uint32_t warp_cells,
-               const ExtPipe *pipe, bool all_rows) {
+               const ExtPipe *pipe, bool all_rows, bool hint_all) {
     if (n == 0) return SWB_OK;
     if (n > 0x7FFFFFF0ull) return set_error(SWB_ERR_TOO_LARGE, "more than 2^31-16 tasks in one batch");
     if (pipe && n > pipe->cap) return set_error(SWB_ERR_INVALID_ARG, "pass larger than its scratch set");
     int rc;
+    if (n <= kExtWarpsMaxTasks && !pipe && !warp_cells && (hint_all || max_q_hint < 0)) {
+        int max_q = max_q_hint;
+        if (max_q < 0) {
+            if ((rc = ensure_dev(ctx, ctx->d_misc, kMiscBytes))) return rc;
+            int *d_max = (int *)((char *)ctx->d_misc.p + 256);
+            SWB_CUDA(cudaMemsetAsync(d_max, 0, sizeof(int), s));
+            max_qlen_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_tasks, (uint32_t)n, d_max);
+            ctx->launches++;
+            SWB_CUDA(cudaGetLastError());
+            SWB_CUDA(cudaMemcpyAsync(&max_q, d_max, sizeof(int), cudaMemcpyDeviceToHost, s));
+            SWB_CUDA(cudaStreamSynchronize(s));
+        }
+        if (max_q <= kWarpMaxQ) return launch_ext_warps(ctx, sc, d_bases, d_tasks, n, d_out, d_cells, s, max_q);
+    }
     // keys, keys2, idx and the sort's temporary storage are used by the
     // launching stream only; the sorted order (idx2) and the bin bounds and
     // claim counters (misc) are read by the bins, one set per pipelined slot.

@@ -94,6 +94,12 @@ constexpr int kSideStreams = 32;   // concurrent bin launches per context
 // that way against 0.36 ms binned; from ~20k mixed-length tasks on, the
 // binned pass is faster.
 constexpr size_t kExtPlainMaxTasks = 16384;
+// Batches up to this many tasks run one warp per extension (launch_ext_warps):
+// they cannot fill the GPU with one thread each and last as long as one task.
+// Host entry, one warp / one thread per task: 1000 tasks of 150 bp reads 255 /
+// 519 us, 4000 532 / 545, 8000 841 / 593; uneven tasks 4000 611 / 1179, 8000
+// 981 / 1234.
+constexpr size_t kExtWarpsMaxTasks = 4096;
 constexpr int kMaxChunks = 16;     // pipelined chunks of one synchronous batch call
 
 // ------------------------------------------------------------ a device arena
@@ -208,6 +214,10 @@ int ensure_host(swb_ctx *ctx, HostBuf &b, size_t bytes);
 // extension (latency), otherwise their length bin's thread-per-task kernel.
 // all_rows: compute every row the reference does, so that `cells` receives the
 // reference's count; else rows that cannot change a result are left out.
+// max_q_hint: at least the longest query of the int32 bin (-1: read back, which
+// synchronises `stream`); hint_all: at least the longest query of all tasks.
+// Passes of up to kExtWarpsMaxTasks tasks whose longest query is known (or
+// read back) run one warp per extension instead of the bins.
 // Pipelined passes: two scratch sets let pass k+1 sort and start its bins
 // while pass k's bins finish.  The caller sizes the scratch with
 // ext_reserve(cap) first and makes `stream` wait for pass k-2 to finish
@@ -221,7 +231,15 @@ int ext_reserve(swb_ctx *ctx, size_t cap);
 int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
                const swb_ext_task *d_tasks, size_t n, swb_ext_result *d_out,
                unsigned long long *d_cells, cudaStream_t stream, int max_q_hint,
-               uint32_t warp_cells = 0, const ExtPipe *pipe = nullptr, bool all_rows = false);
+               uint32_t warp_cells = 0, const ExtPipe *pipe = nullptr, bool all_rows = false,
+               bool hint_all = false);
+
+// Small batches: one warp per extension (max_q: the longest query, at most
+// kExtWarpsMaxLong).
+constexpr int kExtWarpsMaxQ = 255;      // longest query kept in registers
+constexpr int kExtWarpsMaxLong = 4096;
+int launch_ext_warps(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases, const swb_ext_task *d_tasks, size_t n,
+                     swb_ext_result *d_out, unsigned long long *d_cells, cudaStream_t s, int max_q);
 
 // The plain one-launch-per-batch comparator of the extension pass (the same
 // two-row kernel over the batch in input order; no sort, bins or claiming).

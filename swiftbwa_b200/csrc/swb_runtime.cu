@@ -545,12 +545,12 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
     for (size_t k = 0; k < nchunks; ++k) per = std::max(per, cb[k + 1] - cb[k]);
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     struct Part {
-        int code = 0, big_q = 0;
+        int code = 0, big_q = 0, max_q = 0;
         size_t need = 0;
         std::string err;
     };
     std::vector<Part> parts(hw);
-    auto scan_chunk = [&](size_t lo, size_t hi, size_t &need, int &big_q) -> int {
+    auto scan_chunk = [&](size_t lo, size_t hi, size_t &need, int &big_q, int &max_q) -> int {
         const size_t nth = std::min<size_t>(hw, std::max<size_t>(1, (hi - lo) / 16384));
         const size_t sub = (hi - lo + nth - 1) / nth;
         auto work = [&](size_t t) {
@@ -560,6 +560,7 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
             if (a >= b) return;
             int mq, mt;
             if ((pt.code = validate_range(ctx, tasks, a, b, n_bases, &mq, &mt, &pt.err, &pt.code))) return;
+            pt.max_q = mq;
             pt.big_q = ext_big_max_q_range(ctx, tasks, a, b, dsc);
             size_t m = 0;
             for (size_t i = a; i < b; ++i) {
@@ -580,6 +581,7 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
             if (parts[t].code) return set_error(parts[t].code, parts[t].err);
             need = std::max(need, parts[t].need);
             big_q = std::max(big_q, parts[t].big_q);
+            max_q = std::max(max_q, parts[t].max_q);
         }
         return SWB_OK;
     };
@@ -602,8 +604,8 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
     for (size_t k = 0; k < nchunks; ++k) {
         const size_t lo = cb[k], hi = cb[k + 1];
         if (lo >= hi) break;
-        int big_q = 0;
-        if ((rc = scan_chunk(lo, hi, need, big_q))) {
+        int big_q = 0, max_q = 0;
+        if ((rc = scan_chunk(lo, hi, need, big_q, max_q))) {
             // Let the chunks already queued finish before reporting (they write `out`).
             cudaStreamSynchronize(ctx->d2h);
             cudaStreamSynchronize(ctx->stream);
@@ -620,11 +622,14 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
         // k-1's bins may still run while chunk k sorts and starts its own.
         if (k >= 2) SWB_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->chunk_done[k - 2], 0));
         const ExtPipe pipe{(int)(k & 1), per, ctx->d2h};
-        // Small batches take the one-launch form: with too few tasks to fill
+        // Small batches take a one-launch form: with too few tasks to fill
         // the GPU, the sort and the per-bin launches cost more than they save.
-        rc = n_tasks <= kExtPlainMaxTasks
-                 ? launch_ext_plain(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream)
-                 : launch_ext(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, big_q, 0, &pipe, true);
+        if (n_tasks <= kExtWarpsMaxTasks && max_q <= kExtWarpsMaxLong)
+            rc = launch_ext_warps(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, max_q);
+        else if (n_tasks <= kExtPlainMaxTasks)
+            rc = launch_ext_plain(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream);
+        else
+            rc = launch_ext(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, big_q, 0, &pipe, true);
         if (rc) {
             cudaStreamSynchronize(ctx->d2h);
             cudaStreamSynchronize(ctx->stream);
