@@ -584,7 +584,11 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     const cudaStream_t js = pipe ? pipe->join : s;
     ProfScope pass(ctx, s, pipe ? nullptr : "ext_pass", -1);   // fork to join, on the launching stream
     SWB_CUDA(cudaEventRecord(ctx->fork_ev, s));
-    for (int b = 0; b < nbins; ++b) {
+    // The int32 bin and the largest classes first: a bin's blocks get the SMs in
+    // launch order, so the pass ends on the short tasks (131k uneven tasks, smallest first /
+    // largest first: 1676 / 1398 us; 256k 2194 / 1677; 5M 29.8 / 28.9 ms).
+    for (int k = 0; k < nbins; ++k) {
+        const int b = k == 0 ? big : (k & 1 ? bins.n : 0) + bins.n - 1 - (k - 1) / 2;
         cudaStream_t sb = ctx->side[b];
         SWB_CUDA(cudaStreamWaitEvent(sb, ctx->fork_ev, 0));
         if (b < big) {
