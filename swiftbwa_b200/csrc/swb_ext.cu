@@ -59,6 +59,8 @@ constexpr int kFastT = 32;                // threads per block in the shared-mem
 // byte 256, the bins' claim counters from byte 320.
 constexpr size_t kMiscBytes = 512;
 constexpr int kBigT = 64;
+constexpr size_t kSmemPerSm = 227 * 1024;
+constexpr size_t kAheadBlocks = 13;
 // Rows past the query's length that a task is taken to run when it may stop
 // early (sort key only).
 constexpr int kTailRows = 4;
@@ -148,7 +150,7 @@ __global__ void bin_bounds_kernel(const uint32_t *__restrict__ sorted_keys, size
 // qcap: the bin's class bound.  (An instance per bound, with it as a constant,
 // ran 1-4 % slower than this one: 31 instances' code for an inner loop that
 // does not use the bound.)
-template <int T, bool U8, bool ALL>
+template <int T, bool U8, bool ALL, bool AHEAD>
 __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qcap) {
     extern __shared__ uint32_t sm[];
     // Rows: (qcap + 1) words of 2 (int8 scores) or 4 bytes (int16), then
@@ -183,8 +185,8 @@ __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qca
             const int skip = a.skip[ti];
             auto run = [&](auto symc, auto ringc) {
                 constexpr bool kSym = decltype(symc)::value, kRing = decltype(ringc)::value;
-                if constexpr (U8) ext_pair_one<T, kSym, false, kRing, ALL>(a, tk, skip, he16, qc, r, cells);
-                else ext_pair_one<T, kSym, true, kRing, ALL>(a, tk, skip, he32, qc, r, cells);
+                if constexpr (U8) ext_pair_one<T, kSym, false, kRing, ALL, AHEAD>(a, tk, skip, he16, qc, r, cells);
+                else ext_pair_one<T, kSym, true, kRing, ALL, AHEAD>(a, tk, skip, he32, qc, r, cells);
             };
             if (rings && skip == 0) {
                 if (sym) run(std::true_type{}, std::true_type{});
@@ -361,11 +363,11 @@ __global__ void __launch_bounds__(T) ext_plain_kernel(ExtArgs a, size_t n, int q
             const bool sym = a.sc.o_del + a.sc.e_del == a.sc.o_ins + a.sc.e_ins;
             // (No rows left out: unsorted, a warp's tasks rarely all have some.)
             if constexpr (U8) {
-                if (sym) ext_pair_one<T, true, false, false, true>(a, tk, 0, he16, qc, r, cells);
-                else ext_pair_one<T, false, false, false, true>(a, tk, 0, he16, qc, r, cells);
+                if (sym) ext_pair_one<T, true, false, false, true, true>(a, tk, 0, he16, qc, r, cells);
+                else ext_pair_one<T, false, false, false, true, true>(a, tk, 0, he16, qc, r, cells);
             } else {
-                if (sym) ext_pair_one<T, true, true, false, true>(a, tk, 0, he32, qc, r, cells);
-                else ext_pair_one<T, false, true, false, true>(a, tk, 0, he32, qc, r, cells);
+                if (sym) ext_pair_one<T, true, true, false, true, true>(a, tk, 0, he32, qc, r, cells);
+                else ext_pair_one<T, false, true, false, true, true>(a, tk, 0, he32, qc, r, cells);
             }
             a.out[pos] = r;
         }
@@ -390,23 +392,27 @@ const char *bin_name(bool u8, int qcap) {
 
 using FastKernel = void (*)(ExtArgs, int, int);
 
-FastKernel fast_kernel(bool u8, bool all) {
-    if (all) return u8 ? ext_fast_kernel<kFastT, true, true> : ext_fast_kernel<kFastT, false, true>;
-    return u8 ? ext_fast_kernel<kFastT, true, false> : ext_fast_kernel<kFastT, false, false>;
+template <bool U8>
+FastKernel fast_kernel_of(bool all, bool ahead) {
+    if (all) return ahead ? ext_fast_kernel<kFastT, U8, true, true> : ext_fast_kernel<kFastT, U8, true, false>;
+    return ahead ? ext_fast_kernel<kFastT, U8, false, true> : ext_fast_kernel<kFastT, U8, false, false>;
+}
+FastKernel fast_kernel(bool u8, bool all, bool ahead) {
+    return u8 ? fast_kernel_of<true>(all, ahead) : fast_kernel_of<false>(all, ahead);
 }
 
 // Resident one-warp blocks per SM of the shared-memory kernel for a class bound.
-int fast_occupancy(bool u8, bool all, int qcap) {
-    static int cache[4][kExtSmemMaxQ + 1];
+int fast_occupancy(bool u8, bool all, bool ahead, int qcap) {
+    static int cache[8][kExtSmemMaxQ + 1];
     static std::once_flag once;
     std::call_once(once, [] {
         for (auto &row : cache)
             for (int &v : row) v = -1;
     });
-    int &occ = cache[(u8 ? 1 : 0) + (all ? 2 : 0)][qcap];
+    int &occ = cache[(u8 ? 1 : 0) + (all ? 2 : 0) + (ahead ? 4 : 0)][qcap];
     if (occ < 0) {
         int o = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8, all), kFastT, fast_smem_bytes(qcap, u8)) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8, all, ahead), kFastT, fast_smem_bytes(qcap, u8)) !=
             cudaSuccess)
             return -1;
         occ = o < 1 ? 1 : o;
@@ -415,13 +421,19 @@ int fast_occupancy(bool u8, bool all, int qcap) {
 }
 
 int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, cudaStream_t s) {
-    const int occ = fast_occupancy(u8, all, qcap);
+    // Loads a step ahead where latency counts: rows that leave room for fewer
+    // than kAheadBlocks blocks per SM, and passes that do not fill the SMs.
+    // Without / with in every bin / by this rule: 131k uneven tasks 1431 / 1266 /
+    // 1249 us, 5M 28.9 / 26.9 / 26.8 ms; 2M tasks of 150 bp reads 3772 / 3908 /
+    // 3779 us.
+    const bool ahead = n <= (size_t)ctx->sm_count * 20 * kFastT || fast_smem_bytes(qcap, u8) * kAheadBlocks > kSmemPerSm;
+    const int occ = fast_occupancy(u8, all, ahead, qcap);
     if (occ < 0) return check_cuda(cudaGetLastError(), "occupancy query");
     const size_t grid = std::min<size_t>((n + kFastT - 1) / kFastT, (size_t)ctx->sm_count * occ);
     if (grid == 0) return SWB_OK;
     const size_t smem = fast_smem_bytes(qcap, u8);
     ProfScope ps(ctx, s, ctx->prof_on ? bin_name(u8, qcap) : nullptr, kCntExtBin0 + bin);
-    fast_kernel(u8, all)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
+    fast_kernel(u8, all, ahead)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
     return SWB_OK;

@@ -158,7 +158,10 @@ struct RowTrack {
 };
 
 // skip: ext_skip_rows of the task, or 0 (a ring takes 0).
-template <int T, bool SYM, bool W16, bool RING, bool ALL>
+// AHEAD: each lockstep step loads the next column's word and query byte before
+// it computes, which hides the shared-memory latency where few warps are
+// resident and costs a little where many are (ext_fast_kernel's launch chooses).
+template <int T, bool SYM, bool W16, bool RING, bool ALL, bool AHEAD>
 __device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_task &tk, int skip,
                                              RowWord<W16> *he, uint8_t *qc, swb_ext_result &res,
                                              unsigned long long &cells) {
@@ -306,9 +309,7 @@ __device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_tas
             uint32_t jp = (uint32_t)c | ((uint32_t)(c - 1) << 16);
             // One lockstep step: row i's word for column c from slot ls, row i+1's
             // word for column c-1 into slot ss.
-            auto step = [&](int ls, int ss) {
-                const uint32_t wd = he[ls * T];
-                const uint32_t sel = sel_of(qc[ls * T]);
+            auto step_of = [&](uint32_t wd, uint32_t sel, int ss) {
                 const uint32_t Mp = W16 ? __byte_perm(wd, hPrevP, 0x5410) : __byte_perm(wd, hPrevP, 0x5450);   // [H(i-1,c-1), H(i,c-2)]
                 const uint32_t ep = W16 ? __byte_perm(wd, nEPrev, 0x5432) : __byte_perm(wd, nEPrev, 0x5451);   // [E(i,c),     E(i+1,c-1)]
                 const uint32_t sp = lane_score(rt1, sPrev) * 65536u + lane_score(rt0, sel);
@@ -335,9 +336,19 @@ __device__ __forceinline__ void ext_pair_one(const ExtArgs &a, const swb_ext_tas
                 nEPrev = nE;    // low field = row i's E', the high lane's upper bits never reach a word
                 h1p = H;
             };
-            if constexpr (!RING) {
+            auto step = [&](int ls, int ss) { step_of(he[ls * T], sel_of(qc[ls * T]), ss); };
+            if constexpr (!RING && !AHEAD) {
 #pragma unroll 2
                 for (; c < e0; ++c, jp += 0x10001u) step(c, c - 1);
+            } else if constexpr (!RING) {
+                uint32_t wd = he[c * T], q = qc[c * T];
+#pragma unroll 2
+                for (; c < e0; ++c, jp += 0x10001u) {
+                    const uint32_t wn = he[(c + 1) * T], qn = qc[(c + 1) * T];
+                    step_of(wd, sel_of(q), c - 1);
+                    wd = wn;
+                    q = qn;
+                }
             } else {
                 int cs = sl(c);
                 while (c < e0) {
