@@ -27,13 +27,14 @@ constexpr int kNegInf = INT32_MIN / 2;   // GlobalAligner.swift:52
 // CIGARGenerator.generate repeats the DP with the band doubled while the
 // score is below the true score, at most three times (CIGARGenerator.swift:
 // 88-96).  Once the band covers the whole matrix (every row spans all qlen
-// columns: w >= max(qlen, tlen) - 1) a wider band computes the same matrix,
+// columns, w >= max(qlen, tlen) - 1, and so does the first row's
+// initialisation, w >= qlen) a wider band computes the same matrix,
 // score and backpointers, so the attempts left are accounted for -- width,
 // attempt count and their qlen * tlen cells each -- instead of recomputed.
 // Returns true when it did so (the caller stops retrying).
 __device__ __forceinline__ bool nw_skip_covered_retries(int qlen, int tlen, int w, int retries, int &w0,
                                                         swb_global_result &r, unsigned long long &cells) {
-    if (w < imax(qlen, tlen) - 1) return false;
+    if (w < imax(qlen, tlen - 1)) return false;
     const int left = 3 - retries;
     w0 *= 1 << left;
     r.attempts += left;
