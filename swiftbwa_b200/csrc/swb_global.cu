@@ -614,6 +614,233 @@ __global__ void __launch_bounds__(256) global_smem_kernel(GlobalArgs a, const ui
     if ((threadIdx.x & 31) == 0 && cells) atomicAdd(a.cells, cells);
 }
 
+// ------------------------------------------------------------------------
+// One warp per alignment, for the int16-row class (nw_fits_i16, which also
+// keeps every value far from overflow here) in batches that one thread per
+// alignment cannot fill the GPU with.  Lane l keeps columns l*KC .. l*KC+KC-1:
+// H and E of the row above in registers.  Only F runs along a row, and its
+// values need just G = max(diagonal, E) of the columns to the left (opening
+// from an H that F set never beats extending that F), so a row is: diagonal and E
+// per column, a fold of the chunk's G, a five-step shuffle scan with constant
+// decays, and a second pass for F, H and the backpointer codes.  Values are the
+// reference's int32 ones, sentinels included.  A lane's codes of a row are one
+// word, a row one 128-byte store; the traceback walks them with all lanes
+// holding the current row, the next rows loaded ahead.
+// Up to this many alignments: a warp holds one, so about 4,700 are in flight
+// against 44,000 with a thread each, at a third of the throughput but an eighth
+// of the time for one.  Kernel time, warp / thread per alignment, 150 bp reads:
+// band 100, 1k 134 / 674 us, 10k 821 / 717; band 5, 1k 132 / 201, 10k 820 / 254;
+// 100 bp, band 5, 8k 380 / 185; 250 bp, band 100, 1k 320 / 1252.
+constexpr size_t kNwWarpMaxTasks = 4096;
+constexpr int kNwNone = -1500000000;   // below every sentinel-derived value
+
+template <int KC>
+struct NwWarp {
+    int Hc[KC], Ec[KC];   // H and E of the row above, per column
+
+    // One DP attempt with band w (GlobalAligner.swift:26-144); returns h[qlen].
+    __device__ __forceinline__ int dp(const GlobalArgs &a, const swb_global_task &tk, const uint32_t (&sel)[KC], int w,
+                                      uint32_t *z, unsigned long long &cells) {
+        const DevScoring &sc = a.sc;
+        const int lane = threadIdx.x & 31, j0 = lane * KC;
+        const int qlen = tk.qlen, tlen = tk.tlen;
+        const int eDel = sc.e_del, eIns = sc.e_ins, oeDel = sc.o_del + eDel, oeIns = sc.o_ins + eIns;
+        const int initEnd = imin(w, qlen);
+#pragma unroll
+        for (int k = 0; k < KC; ++k) {                                           // :75-84
+            const int j1 = j0 + k + 1;
+            Hc[k] = j1 <= initEnd ? 0 - (sc.o_ins + eIns * j1) : kNegInf;
+            Ec[k] = kNegInf;
+        }
+        auto tload = [&](int r) -> uint32_t {
+            return r < tlen ? span_base(a.bases, a.pac, tk.t_off, r, tlen, tk.flags, true) : 4u;
+        };
+        uint32_t tcur = tload(lane), tnext = tload(32 + lane);   // 32 target rows per load, a block ahead
+        unsigned long long n = 0;
+        for (int i = 0; i < tlen; ++i) {                                         // :89-142
+            if (i > 0 && (i & 31) == 0) {
+                tcur = tnext;
+                tnext = tload(i + 32 + lane);
+            }
+            const RowTable rt = row_table(sc, __shfl_sync(0xFFFFFFFFu, tcur, i & 31));
+            const int beg = imax(0, i - w), end = (int)min((long long)qlen, (long long)i + w + 1);
+            n += (unsigned long long)imax(end - beg, 0);
+            const int hBeg = beg == 0 ? 0 - (oeDel + eDel * i) : kNegInf;
+            int dg = __shfl_up_sync(0xFFFFFFFFu, Hc[KC - 1], 1);                 // H(i-1, j-1) of the first column
+            if (lane == 0) dg = i == 0 ? 0 : 0 - (oeDel + eDel * (i - 1));
+            const int f0 = imax(kNegInf - eIns, hBeg - oeIns);                   // F of column beg
+            const bool f0Ext = kNegInf - eIns >= hBeg - oeIns;
+            int G[KC];
+            uint32_t code[KC];
+            int agg = kNwNone;
+#pragma unroll
+            for (int k = 0; k < KC; ++k) {
+                const int j = j0 + k;
+                const bool in = j >= beg && j < end;
+                const int up = Hc[k];
+                bool eExt, keep;
+                const int ev = __vibmax_s32(Ec[k] - eDel, up - oeDel, &eExt);     // extend unless open > extend
+                G[k] = __vibmax_s32(dg + (int)prmt(rt.lo, rt.hi, sel[k]), ev, &keep);   // from E when E > H
+                code[k] = (eExt ? 1u : 0u) | (keep ? 0u : 4u);
+                if (in) Ec[k] = ev;
+                dg = up;
+                if (j == beg) agg = f0;
+                if (in) agg = imax(agg - eIns, G[k] - oeIns);
+            }
+            int incl = agg;
+#pragma unroll
+            for (int d = 0; d < 5; ++d) {
+                const int o = __shfl_up_sync(0xFFFFFFFFu, incl, 1 << d);
+                if (lane >= 1 << d) incl = imax(incl, o - ((eIns * KC) << d));
+            }
+            int f = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
+            bool fExt = false;                                                   // (the first column's comes by ballot)
+            uint32_t word = 0;
+#pragma unroll
+            for (int k = 0; k < KC; ++k) {
+                const int j = j0 + k;
+                if (j == beg) {
+                    f = f0;
+                    fExt = f0Ext;
+                }
+                const bool in = j >= beg && j < end;
+                bool keep, ext;
+                const int H = __vibmax_s32(G[k], f, &keep);                      // from F when F > H
+                const uint32_t c = code[k] | (fExt ? 2u : 0u) | (keep ? 0u : 8u);
+                f = __vibmax_s32(f - eIns, H - oeIns, &ext);
+                fExt = ext;
+                if (in) {
+                    Hc[k] = H;
+                    word |= c << (4 * k);
+                }
+            }
+            const unsigned left = __ballot_sync(0xFFFFFFFFu, fExt) << 1;
+            if (j0 > beg && j0 < end && ((left >> lane) & 1u)) word |= 2u;
+            z[(size_t)i * 32] = word;
+        }
+        if (lane == 0) cells += n;
+        int v = 0;
+#pragma unroll
+        for (int k = 0; k < KC; ++k)
+            if (k == (qlen - 1) % KC) v = Hc[k];
+        return __shfl_sync(0xFFFFFFFFu, v, (qlen - 1) / KC);                     // :144
+    }
+
+    // GlobalAligner.swift:160-232 (global_traceback), run by the whole warp;
+    // lane 0 writes the ops.
+    __device__ __forceinline__ int traceback(const uint32_t *z, int qlen, int tlen, int w, int nCol,
+                                             uint32_t *out) const {
+        const int lane = threadIdx.x & 31;
+        CigarOut c{out};
+        auto put = [&](uint32_t o) {
+            if (o == c.op) {
+                ++c.len;
+                return;
+            }
+            if (c.len) {
+                if (lane == 0) c.p[c.n] = (c.len << 4) | c.op;
+                ++c.n;
+            }
+            c.op = o;
+            c.len = 1;
+        };
+        int i = tlen - 1, j = qlen - 1, state = 0;
+        auto zload = [&](int r) -> uint32_t { return r >= 0 ? z[(size_t)r * 32] : 0u; };
+        uint32_t r0 = zload(i), r1 = zload(i - 1), r2 = zload(i - 2), r3 = zload(i - 3), r4 = zload(i - 4);
+        auto row_up = [&]() {
+            --i;
+            r0 = r1;
+            r1 = r2;
+            r2 = r3;
+            r3 = r4;
+            r4 = zload(i - 4);
+        };
+        while (i >= 0 || j >= 0) {
+            if (i < 0) { put(1u); --j; continue; }
+            if (j < 0) { put(2u); --i; continue; }
+            const int col = j - imax(0, i - w);
+            if (!(col >= 0 && col < nCol)) break;
+            const uint32_t d = (__shfl_sync(0xFFFFFFFFu, r0, j / KC) >> (4 * (j % KC))) & 0xFu;
+            if (state == 0) {
+                const uint32_t hDir = d >> 2;
+                if (hDir == 0) { put(0u); --j; row_up(); }
+                else state = hDir == 1 ? 1 : 2;
+            } else if (state == 1) {
+                put(2u);
+                if ((d & 1u) == 0) state = 0;
+                row_up();
+            } else {
+                put(1u);
+                if ((d & 2u) == 0) state = 0;
+                --j;
+            }
+        }
+        if (lane == 0) c.finish();
+        return lane == 0 ? c.n : 0;
+    }
+};
+
+// Sorted int16-row alignments order[begin, begin + count), claimed one per warp.
+template <int KC>
+__global__ void __launch_bounds__(128, KC <= 5 ? 8 : 6) global_warp_kernel(GlobalArgs a, const uint32_t *__restrict__ order,
+                                                                          size_t begin, uint32_t count, uint32_t *claim,
+                                                                          uint32_t *zbase, int zrows) {
+    const int lane = threadIdx.x & 31;
+    uint32_t *z = zbase + ((size_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * zrows * 32 + lane;
+    unsigned long long cells = 0;
+    for (;;) {
+        uint32_t p = 0;
+        if (lane == 0) p = atomicAdd(claim, 1u);
+        p = __shfl_sync(0xFFFFFFFFu, p, 0);
+        if (p >= count) break;
+        const size_t k = order[begin + p];
+        const swb_global_task tk = a.tasks[k];
+        swb_global_result r{0, 0, tk.w, 1, a.cigar_off[k]};
+        const int qlen = tk.qlen, tlen = tk.tlen;
+        if (qlen > 0 && tlen > 0) {                                      // :29-31
+            uint32_t sel[KC];   // row_score's byte selector of the query code
+#pragma unroll
+            for (int c = 0; c < KC; ++c) {
+                const int j = lane * KC + c;
+                sel[c] = (j < qlen ? span_base(a.bases, a.pac, tk.q_off, j, qlen, tk.flags, false) : 4u) * 0x1111u + 0x8880u;
+            }
+            NwWarp<KC> nw;
+            int w0 = tk.w;
+            int w = imax(w0, abs(qlen - tlen));                          // :47
+            int nCol = (int)min((long long)qlen, 2ll * w + 1);           // :48
+            int score = nw.dp(a, tk, sel, w, z, cells);
+            if (tk.flags & SWB_GLB_RETRY) {                              // CIGARGenerator.swift:88-96
+                int retries = 0;
+                while (score < tk.true_score && retries < 3) {
+                    unsigned long long skipped = 0;
+                    const bool done = nw_skip_covered_retries(qlen, tlen, w, retries, w0, r, skipped);
+                    if (lane == 0) cells += skipped;
+                    if (done) break;
+                    w0 *= 2;
+                    ++retries;
+                    r.attempts++;
+                    w = imax(w0, abs(qlen - tlen));
+                    nCol = (int)min((long long)qlen, 2ll * w + 1);
+                    score = nw.dp(a, tk, sel, w, z, cells);
+                }
+            }
+            r.score = score;
+            r.w_used = w0;
+            r.n_cigar = nw.traceback(z, qlen, tlen, w, nCol, a.cigar + r.cigar_off);
+        }
+        if (lane == 0) a.res[k] = r;
+        __syncwarp();
+    }
+    for (int o = 16; o > 0; o >>= 1) cells += __shfl_down_sync(0xFFFFFFFFu, cells, o);
+    if (lane == 0 && cells) atomicAdd(a.cells, cells);
+}
+
+using NwWarpKernel = void (*)(GlobalArgs, const uint32_t *, size_t, uint32_t, uint32_t *, uint32_t *, int);
+NwWarpKernel nw_warp_kernel(int qcap) {
+    return qcap <= 128 ? global_warp_kernel<4> : qcap <= 160 ? global_warp_kernel<5>
+         : qcap <= 192 ? global_warp_kernel<6> : global_warp_kernel<8>;
+}
+
 __global__ void cigar_offsets_kernel(const swb_global_task *__restrict__ tasks, size_t n,
                                      unsigned long long *__restrict__ lens) {
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -663,8 +890,19 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         size_t smem = 0, nslots = 0;
     } cfg[2];   // [0] int32 rows, [1] int16 rows
     size_t z_bytes = 0;
-    int qcap = 0;
+    int qcap = 0, warp_grid = 0;
     const size_t n_small_of[2] = {shape.n_small - shape.n_small16, shape.n_small16};
+    const int zrows = imax(shape.small_t, 1);
+    if (shape.n_small16 > 0 && shape.n_small16 <= kNwWarpMaxTasks) {
+        // One warp per alignment: resident blocks of four, each warp with its
+        // own backpointer rows.
+        int occ = 0;
+        SWB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, nw_warp_kernel(imax(shape.small_q, 1)), 128, 0));
+        warp_grid = (int)std::min<size_t>((size_t)ctx->sm_count * imax(occ, 1), (shape.n_small16 + 3) / 4);
+        while (warp_grid > 1 && (size_t)warp_grid * 4 * zrows * 128 > avail0) warp_grid /= 2;
+        z_bytes = ((size_t)warp_grid * 4 * zrows * 128 + 1023) & ~(size_t)1023;
+        if (z_bytes > avail0) warp_grid = 0, z_bytes = 0;
+    }
     if (shape.n_small > 0) {
         qcap = imax(shape.small_q, 1);
         int sm_bytes = 0, blk_bytes = 0;
@@ -673,7 +911,7 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         const size_t per_slot = (size_t)imax(shape.small_t, 1) * (size_t)((qcap + 7) >> 3) * 4;
         size_t max_slots = 0;
         for (int v = 0; v < 2; ++v) {
-            if (n_small_of[v] == 0) continue;
+            if (n_small_of[v] == 0 || (v && warp_grid)) continue;
             const size_t per_thread = (size_t)(qcap + 1) * (v ? 4 : 8) + (size_t)((qcap + 7) & ~7);
             int best = 0, T = 0;
             for (int t = 32; t <= 256; t += 32) {
@@ -696,7 +934,7 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
             if (v) SWB_CUDA(cudaFuncSetAttribute(global_smem_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
             else SWB_CUDA(cudaFuncSetAttribute(global_smem_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
         }
-        z_bytes = (max_slots * per_slot + 1023) & ~(size_t)1023;
+        z_bytes = std::max(z_bytes, (max_slots * per_slot + 1023) & ~(size_t)1023);
         if (z_bytes > avail0) return set_error(SWB_ERR_OOM, "global alignment scratch does not fit the memory budget");
     }
     // Global-scratch kernel for longer queries.
@@ -726,7 +964,10 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     for (int v = 1; v >= 0; --v) {
         if (n_small_of[v] == 0) continue;
         const SmemCfg &c = cfg[v];
-        if (v)
+        if (v && warp_grid)
+            nw_warp_kernel(qcap)<<<(unsigned)warp_grid, 128, 0, st>>>(a, order, begin_of[v], (uint32_t)n_small_of[v],
+                                                                     claim + v, (uint32_t *)ctx->d_scratch.p, zrows);
+        else if (v)
             global_smem_kernel<true><<<(unsigned)c.grid, c.T, c.smem, st>>>(
                 a, order, begin_of[v], (uint32_t)n_small_of[v], claim + v, (uint32_t *)ctx->d_scratch.p, c.nslots, qcap);
         else
