@@ -522,8 +522,10 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
     // the batch, so each chunk's copy (≈2.6 ns per config-1 task) ends within
     // the kernels of the one before (≈3.6 ns per task) and the GPU waits only
     // for the first, then two short chunks (6 % and 3 %) so that the last
-    // pass and its copy back are short.  Smaller batches: up to eight equal
-    // chunks of at least 512K tasks.  The host checks chunk k (spans, the
+    // pass and its copy back are short.  Smaller batches: equal chunks of about
+    // 256K tasks, at most four, or more of at least 512K (up to eight), so that
+    // copies overlap the kernels from half a million tasks on (a chunk still
+    // holds more tasks than the GPU lanes).  The host checks chunk k (spans, the
     // bases prefix it needs, the longest query of the int32 bin) while the
     // GPU works on the chunks before it; chunk k starts once the prefix of
     // `bases` its tasks reference is on the device.
@@ -535,7 +537,9 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
             for (double f : kGrow) cb.push_back((size_t)(f * (double)n_tasks));
             cb.push_back(n_tasks);
         } else {
-            const size_t m = std::min<size_t>(8, std::max<size_t>(1, n_tasks / kMinChunk)), p = (n_tasks + m - 1) / m;
+            const size_t few = std::min<size_t>(4, (n_tasks + kMinChunk / 4) / (kMinChunk / 2));
+            const size_t m = std::min<size_t>(8, std::max<size_t>({1, few, n_tasks / kMinChunk}));
+            const size_t p = (n_tasks + m - 1) / m;
             for (size_t k = 1; k <= m; ++k) cb.push_back(std::min(n_tasks, k * p));
         }
     }
