@@ -644,9 +644,12 @@ int ext_big_max_q_range(const swb_ctx *ctx, const swb_ext_task *tasks, size_t lo
 // The plain comparator (see ext_plain_kernel): one launch of the two-row code
 // over the batch in input order, then the int32 kernels over the tasks it
 // cannot take.  The batch's shape (row length and width) is read back from
-// the device, which synchronises `s` once.
+// the device, which synchronises `s` once, unless the caller knows that the
+// two-row code takes every task: pair_q >= 0, their longest query, and need16,
+// whether one needs int16 rows.
 int launch_ext_plain(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases, const swb_ext_task *d_tasks,
-                     size_t n, swb_ext_result *d_out, unsigned long long *d_cells, cudaStream_t s) {
+                     size_t n, swb_ext_result *d_out, unsigned long long *d_cells, cudaStream_t s, int pair_q,
+                     bool need16) {
     if (n == 0) return SWB_OK;
     if (n > 0x7FFFFFF0ull) return set_error(SWB_ERR_TOO_LARGE, "more than 2^31-16 tasks in one batch");
     int rc;
@@ -656,19 +659,21 @@ int launch_ext_plain(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     PlainShape *shape = (PlainShape *)(misc + kPlainShapeOff);
     uint32_t *claim = (uint32_t *)(misc + 320);
     uint32_t *order = (uint32_t *)ctx->d_idx2.p;
-    SWB_CUDA(cudaMemsetAsync(misc, 0, kMiscBytes, s));
     const int pair_ok = sc.o_del + sc.e_del <= 32767 && sc.o_ins + sc.e_ins <= 32767;
-    const unsigned tb = 256;
-    {
-        ProfScope ps(ctx, s, "ext_plain_scan", -1);
-        ext_plain_scan_kernel<<<(unsigned)((n + tb - 1) / tb), tb, 0, s>>>(d_tasks, n, sc.max_mat, pair_ok, bin_start,
-                                                                            order, shape);
+    PlainShape sh{imax(pair_q, 1), need16 ? 1 : 0, 0};
+    if (pair_q < 0 || !pair_ok) {
+        SWB_CUDA(cudaMemsetAsync(misc, 0, kMiscBytes, s));
+        const unsigned tb = 256;
+        {
+            ProfScope ps(ctx, s, "ext_plain_scan", -1);
+            ext_plain_scan_kernel<<<(unsigned)((n + tb - 1) / tb), tb, 0, s>>>(d_tasks, n, sc.max_mat, pair_ok, bin_start,
+                                                                                order, shape);
+        }
+        ctx->launches++;
+        SWB_CUDA(cudaGetLastError());
+        SWB_CUDA(cudaMemcpyAsync(&sh, shape, sizeof(sh), cudaMemcpyDeviceToHost, s));
+        SWB_CUDA(cudaStreamSynchronize(s));
     }
-    ctx->launches++;
-    SWB_CUDA(cudaGetLastError());
-    PlainShape sh{};
-    SWB_CUDA(cudaMemcpyAsync(&sh, shape, sizeof(sh), cudaMemcpyDeviceToHost, s));
-    SWB_CUDA(cudaStreamSynchronize(s));
     if (sh.big_max_q > kMaxLen) return set_error(SWB_ERR_TOO_LARGE, "query longer than 65535 bases");
     ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, order, bin_start, d_cells, claim};
     if (sh.pair_max_q > 0) {

@@ -153,6 +153,7 @@ struct swb_ctx {
     unsigned long long last_cells = 0;
     // per-kernel profiling
     unsigned long long *d_counters = nullptr;   // swb::kNumCounters cells counters
+    unsigned long long *h_counters = nullptr;   // their pinned copy of the last synchronous call
     swb::ExtBins ext_bins;   // extension length classes (swb_set_ext_bins / swb_tune_ext_bins)
     bool prof_on = false;
     struct ProfRec {
@@ -243,9 +244,13 @@ int launch_ext_warps(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
 
 // The plain one-launch-per-batch comparator of the extension pass (the same
 // two-row kernel over the batch in input order; no sort, bins or claiming).
-// Reads the batch's shape back from the device: synchronises `stream` once.
+// Reads the batch's shape back from the device, which synchronises `stream`
+// once, unless the caller gives it: pair_q, the longest query, when no query is
+// above kExtSmemMaxQ and every score fits int16, and need16, whether some do
+// not fit a byte.
 int launch_ext_plain(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases, const swb_ext_task *d_tasks,
-                     size_t n, swb_ext_result *d_out, unsigned long long *d_cells, cudaStream_t stream);
+                     size_t n, swb_ext_result *d_out, unsigned long long *d_cells, cudaStream_t stream, int pair_q = -1,
+                     bool need16 = false);
 
 // Banded global + traceback (kernel 2).  Tasks with qlen <= kGlobalSmemMaxQ
 // run in the shared-memory kernel, longer ones in the global-scratch kernel;

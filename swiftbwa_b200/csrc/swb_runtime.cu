@@ -267,20 +267,21 @@ struct Timer {
         SWB_CUDA(cudaEventRecord(ctx->ev_start, ctx->stream));
         return SWB_OK;
     }
+    // The counters come back with the results (into pinned words), not by a
+    // copy of their own after them.
     int end() {
         SWB_CUDA(cudaEventRecord(ctx->ev_stop, ctx->stream));
+        SWB_CUDA(cudaMemcpyAsync(ctx->h_counters, d_cells, sizeof(unsigned long long) * kNumCounters,
+                                 cudaMemcpyDeviceToHost, ctx->stream));
         return SWB_OK;
     }
     // After the stream synchronised.
     void collect() {
         float ms = 0.f;
         if (cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop) == cudaSuccess) ctx->last_ms = ms;
-        unsigned long long c[kNumCounters] = {0};
-        if (cudaMemcpy(c, d_cells, sizeof(c), cudaMemcpyDeviceToHost) == cudaSuccess) {
-            unsigned long long sum = 0;
-            for (int k = 0; k < kNumCounters; ++k) sum += c[k];
-            ctx->last_cells = sum;
-        }
+        unsigned long long sum = 0;
+        for (int k = 0; k < kNumCounters; ++k) sum += ctx->h_counters[k];
+        ctx->last_cells = sum;
     }
 };
 
@@ -425,6 +426,7 @@ int swb_init(int device, size_t mem_budget_bytes, swb_ctx **out) {
     cudaError_t e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&ctx->d_counters, sizeof(unsigned long long) * kNumCounters);
     if (e == cudaSuccess) e = cudaMemset(ctx->d_counters, 0, sizeof(unsigned long long) * kNumCounters);
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_counters, sizeof(unsigned long long) * kNumCounters);
     for (int k = 0; k < kSideStreams && e == cudaSuccess; ++k) {
         e = cudaStreamCreateWithFlags(&ctx->side[k], cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join_ev[k], cudaEventDisableTiming);
@@ -456,6 +458,7 @@ void swb_destroy(swb_ctx *ctx) {
     for (DevBuf *b : bufs) free_buf(ctx, *b);
     if (ctx->d_pac && ctx->pac_owned) cudaFree(ctx->d_pac);
     if (ctx->d_counters) cudaFree(ctx->d_counters);
+    if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     if (ctx->h_in.p) cudaFreeHost(ctx->h_in.p);
     if (ctx->h_out.p) cudaFreeHost(ctx->h_out.p);
@@ -550,11 +553,12 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     struct Part {
         int code = 0, big_q = 0, max_q = 0;
+        long long max_score = 0;   // bound of any H; above int16 where one may be
         size_t need = 0;
         std::string err;
     };
     std::vector<Part> parts(hw);
-    auto scan_chunk = [&](size_t lo, size_t hi, size_t &need, int &big_q, int &max_q) -> int {
+    auto scan_chunk = [&](size_t lo, size_t hi, size_t &need, int &big_q, int &max_q, long long &max_score) -> int {
         const size_t nth = std::min<size_t>(hw, std::max<size_t>(1, (hi - lo) / 16384));
         const size_t sub = (hi - lo + nth - 1) / nth;
         auto work = [&](size_t t) {
@@ -569,6 +573,8 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
             size_t m = 0;
             for (size_t i = a; i < b; ++i) {
                 const swb_ext_task &tk = tasks[i];
+                if (tk.qlen > 0 && tk.tlen > 0)
+                    pt.max_score = std::max(pt.max_score, tk.h0 < 0 ? 1ll << 40 : (long long)tk.h0 + (long long)tk.qlen * dsc.max_mat);
                 if (tk.qlen > 0) m = std::max<size_t>(m, tk.q_off + (size_t)tk.qlen);
                 if (tk.tlen > 0 && !(tk.flags & SWB_T_FROM_REF)) m = std::max<size_t>(m, tk.t_off + (size_t)tk.tlen);
             }
@@ -586,6 +592,7 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
             need = std::max(need, parts[t].need);
             big_q = std::max(big_q, parts[t].big_q);
             max_q = std::max(max_q, parts[t].max_q);
+            max_score = std::max(max_score, parts[t].max_score);
         }
         return SWB_OK;
     };
@@ -609,7 +616,8 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
         const size_t lo = cb[k], hi = cb[k + 1];
         if (lo >= hi) break;
         int big_q = 0, max_q = 0;
-        if ((rc = scan_chunk(lo, hi, need, big_q, max_q))) {
+        long long max_score = 0;
+        if ((rc = scan_chunk(lo, hi, need, big_q, max_q, max_score))) {
             // Let the chunks already queued finish before reporting (they write `out`).
             cudaStreamSynchronize(ctx->d2h);
             cudaStreamSynchronize(ctx->stream);
@@ -631,7 +639,8 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
         if (n_tasks <= kExtWarpsMaxTasks && max_q <= kExtWarpsMaxLong)
             rc = launch_ext_warps(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, max_q);
         else if (n_tasks <= kExtPlainMaxTasks)
-            rc = launch_ext_plain(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream);
+            rc = launch_ext_plain(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream,
+                                  max_q <= kExtSmemMaxQ && max_score <= 32000 ? max_q : -1, max_score > 255);
         else
             rc = launch_ext(ctx, dsc, d_b, d_t + lo, hi - lo, d_o + lo, tm.d_cells, ctx->stream, big_q, 0, &pipe, true);
         if (rc) {
