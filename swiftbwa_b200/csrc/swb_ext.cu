@@ -420,7 +420,9 @@ int fast_occupancy(bool u8, bool all, bool ahead, int qcap) {
     return occ;
 }
 
-int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, cudaStream_t s) {
+// n: the pass's tasks; in_bin: at least the bin's.
+int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, size_t in_bin,
+                cudaStream_t s) {
     // Loads a step ahead where latency counts: rows that leave room for fewer
     // than kAheadBlocks blocks per SM, and passes that do not fill the SMs.
     // Without / with in every bin / by this rule: 131k uneven tasks 1431 / 1266 /
@@ -429,7 +431,7 @@ int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int 
     const bool ahead = n <= (size_t)ctx->sm_count * 20 * kFastT || fast_smem_bytes(qcap, u8) * kAheadBlocks > kSmemPerSm;
     const int occ = fast_occupancy(u8, all, ahead, qcap);
     if (occ < 0) return check_cuda(cudaGetLastError(), "occupancy query");
-    const size_t grid = std::min<size_t>((n + kFastT - 1) / kFastT, (size_t)ctx->sm_count * occ);
+    const size_t grid = std::min<size_t>((in_bin + kFastT - 1) / kFastT, (size_t)ctx->sm_count * occ);
     if (grid == 0) return SWB_OK;
     const size_t smem = fast_smem_bytes(qcap, u8);
     ProfScope ps(ctx, s, ctx->prof_on ? bin_name(u8, qcap) : nullptr, kCntExtBin0 + bin);
@@ -564,11 +566,16 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
 
-    // Global-scratch bin: size its scratch from the longest query in it.
+    // Global-scratch bin: size its scratch from the longest query in it.  When
+    // that has to be read back, the bins' sizes come along: empty ones are not
+    // launched and the others get no more blocks than they have work for.
     int max_q = max_q_hint;
-    if (max_q < 0) {
-        SWB_CUDA(cudaMemcpyAsync(&max_q, big_max_q, sizeof(int), cudaMemcpyDeviceToHost, s));
+    uint32_t shape[(256 + sizeof(int)) / 4];
+    const bool sized = max_q < 0;
+    if (sized) {
+        SWB_CUDA(cudaMemcpyAsync(shape, misc, sizeof(shape), cudaMemcpyDeviceToHost, s));
         SWB_CUDA(cudaStreamSynchronize(s));
+        max_q = (int)shape[256 / 4];
     }
     if (max_q > kMaxLen) return set_error(SWB_ERR_TOO_LARGE, "query longer than 65535 bases");
     const size_t nslots = (size_t)ctx->sm_count * 4 * kBigT;
@@ -601,11 +608,13 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     // largest first: 1676 / 1398 us; 256k 2194 / 1677; 5M 29.8 / 28.9 ms).
     for (int k = 0; k < nbins; ++k) {
         const int b = k == 0 ? big : (k & 1 ? bins.n : 0) + bins.n - 1 - (k - 1) / 2;
+        if (b == big ? max_q <= 0 : sized && shape[b + 1] == shape[b]) continue;
         cudaStream_t sb = ctx->side[b];
         SWB_CUDA(cudaStreamWaitEvent(sb, ctx->fork_ev, 0));
         if (b < big) {
-            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], n, sb))) return rc;
-        } else if (max_q > 0) {
+            const size_t in_bin = sized ? shape[b + 1] - shape[b] : n;
+            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], n, in_bin, sb))) return rc;
+        } else {
             ProfScope ps(ctx, sb, "ext_big_i32", kCntExtBin0 + big);
             ext_warp_kernel<<<(unsigned)wblocks, wwarps * 32, wwarps * wstride, sb>>>(a, big, wq);
             ctx->launches++;
