@@ -400,14 +400,19 @@ struct ZRow {
 
 // One lockstep step at column c (both lanes): row i at c, row i+1 at c-1.
 // Returns the two backpointer codes; stores row i+1's word c.
+// wdn, qn: the word and query byte of the step, loaded during the one before
+// (few warps are resident, so shared-memory latency counts).
 struct NwLane2 {
-    uint32_t h, hp2, e, f, wdp, selp;
+    uint32_t h, hp2, e, f, wdp, selp, wdn, qn;
 };
 __device__ __forceinline__ void nw_both(const NwPairConsts &k, const RowTable &rt0, const RowTable &rt1,
                                         uint32_t *__restrict__ he, const uint8_t *__restrict__ qs, int T, int c,
-                                        NwLane2 &st, uint32_t &code0, uint32_t &code1) {
-    const uint32_t wd = he[(c + 1) * T];                          // [H(i-1,c) | E(i-1,c)]
-    const uint32_t sel = nw_sel(qs[c * T]);
+                                        int qlast, NwLane2 &st, uint32_t &code0, uint32_t &code1) {
+    const uint32_t wd = st.wdn;                                   // [H(i-1,c) | E(i-1,c)]
+    const uint32_t sel = nw_sel(st.qn);
+    const int cn = imin(c + 1, qlast);
+    st.wdn = he[(cn + 1) * T];
+    st.qn = qs[cn * T];
     const uint32_t DG = __byte_perm(st.wdp, st.hp2, 0x5410);      // [H(i-1,c-1), H(i,c-2)]
     const uint32_t UH = __byte_perm(wd, st.h, 0x5410);            // [H(i-1,c),   H(i,c-1)]
     const uint32_t UE = __byte_perm(wd, st.e, 0x5432);            // [E(i-1,c),   E(i,c-1)]
@@ -449,7 +454,7 @@ __device__ int global_dp_pair16(const DevScoring &sc, uint32_t *__restrict__ he,
         ZRow z0{z0w, ns}, z1{z1w, ns};
         // Lane 0 state: H of row i at column beg0-1 is hBeg0 (the reference's h[beg0]); F starts at -inf.
         NwLane2 st{(uint32_t)hBeg0 & 0xFFFFu, (uint32_t)hBeg0 & 0xFFFFu, 0u, (uint32_t)(uint16_t)kNeg,
-                   he[beg0 * T], 0u};
+                   he[beg0 * T], 0u, he[(beg0 + 1) * T], qs[beg0 * T]};
         uint32_t code0, code1;
         if (!pair) {                                   // the last row alone: it stores its own words
             for (int c = beg0; c < end0; ++c) {
@@ -470,7 +475,7 @@ __device__ int global_dp_pair16(const DevScoring &sc, uint32_t *__restrict__ he,
         int c = beg0;
         const int aEnd = imin(beg1, end0 - 1);
         for (; c <= aEnd; ++c) {
-            nw_both(k, rt0, rt1, he, qs, T, c, st, code0, code1);
+            nw_both(k, rt0, rt1, he, qs, T, c, qlen - 1, st, code0, code1);
             z0.put(c, code0, end0 - 1);
         }
         // Lane 1: H at beg1-1 is hBeg1, F is -inf; the reference's h[beg1] = hBeg1.
@@ -479,7 +484,7 @@ __device__ int global_dp_pair16(const DevScoring &sc, uint32_t *__restrict__ he,
         reinterpret_cast<int16_t *>(he + beg1 * T)[0] = (int16_t)hBeg1;
         // Both rows, columns c .. end0-1 (row i+1 at c-1): first up to a multiple of 8.
         for (; c < end0 && (c & 7); ++c) {
-            nw_both(k, rt0, rt1, he, qs, T, c, st, code0, code1);
+            nw_both(k, rt0, rt1, he, qs, T, c, qlen - 1, st, code0, code1);
             z0.put(c, code0, end0 - 1);
             z1.put(c - 1, code1, end1 - 1);
         }
@@ -487,13 +492,13 @@ __device__ int global_dp_pair16(const DevScoring &sc, uint32_t *__restrict__ he,
         // completes word c/8 - 1 (nibble 7, column c-1) then fills nibbles 0..6 of word c/8.
         for (; c + 8 <= end0; c += 8) {
             uint32_t w0 = 0, w1;
-            nw_both(k, rt0, rt1, he, qs, T, c, st, code0, code1);
+            nw_both(k, rt0, rt1, he, qs, T, c, qlen - 1, st, code0, code1);
             w0 |= code0;
             z1w[(size_t)((c >> 3) - 1) * ns] = z1.acc | (code1 << 28);
             w1 = 0;
 #pragma unroll
             for (int s2 = 1; s2 < 8; ++s2) {
-                nw_both(k, rt0, rt1, he, qs, T, c + s2, st, code0, code1);
+                nw_both(k, rt0, rt1, he, qs, T, c + s2, qlen - 1, st, code0, code1);
                 w0 |= code0 << (4 * s2);
                 w1 |= code1 << (4 * (s2 - 1));
             }
@@ -501,7 +506,7 @@ __device__ int global_dp_pair16(const DevScoring &sc, uint32_t *__restrict__ he,
             z1.acc = w1;
         }
         for (; c < end0; ++c) {
-            nw_both(k, rt0, rt1, he, qs, T, c, st, code0, code1);
+            nw_both(k, rt0, rt1, he, qs, T, c, qlen - 1, st, code0, code1);
             z0.put(c, code0, end0 - 1);
             z1.put(c - 1, code1, end1 - 1);
         }
