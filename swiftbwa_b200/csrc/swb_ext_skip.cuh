@@ -85,7 +85,10 @@ __device__ __forceinline__ int ext_match_len(const swb_ext_task &tk, const uint8
 // First rows a task leaves out: up to its first mismatch less the lookback.
 __device__ __forceinline__ int ext_skip_rows(const swb_ext_task &tk, const DevScoring &sc,
                                              const uint8_t *__restrict__ bases, const uint8_t *__restrict__ pac) {
-    if (sc.a <= 0 || tk.h0 <= 0 || tk.w < 1 || tk.qlen <= 0 || tk.tlen <= 0) return 0;
+    constexpr int kMost = 1 << 20;   // keeps the sums below within int32
+    if (sc.a <= 0 || tk.h0 <= 0 || tk.h0 > (1 << 29) || tk.w < 1 || tk.qlen <= 0 || tk.tlen <= 0 || sc.o_ins > kMost ||
+        sc.e_ins > kMost || sc.o_del > kMost || sc.e_del > kMost)
+        return 0;
     return imax(ext_match_len(tk, bases, pac) - ext_lookback(sc), 0);
 }
 
