@@ -15,6 +15,8 @@
 //            them back to BWT coordinates (:133-163), in candidate order.
 #include <algorithm>
 #include <string>
+#include <cstring>
+#include <thread>
 #include <vector>
 
 #include <cub/device/device_scan.cuh>
@@ -185,6 +187,18 @@ __global__ void rescue_apply_kernel(RescueArgs a, const swb_local_result *__rest
     n_out[j] = k;
 }
 
+// Packs every job's regions in job order (off = exclusive sum of n_out), so that
+// only those cross to the host: the output has four entries per template
+// region, and a job fills one or two of them.
+__global__ void rescue_pack_kernel(const swb_rescue_job *__restrict__ jobs, size_t n_jobs,
+                                   const swb_rescued *__restrict__ regions, const uint32_t *__restrict__ n_out,
+                                   const unsigned long long *__restrict__ off, swb_rescued *__restrict__ out) {
+    const size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (j >= n_jobs) return;
+    const swb_rescued *src = regions + 4 * (size_t)jobs[j].tmpl_off;
+    for (uint32_t k = 0; k < n_out[j]; ++k) out[off[j] + k] = src[k];
+}
+
 inline size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace
@@ -324,11 +338,53 @@ extern "C" int swb_mate_rescue(swb_ctx *ctx, const swb_scoring *sc, const uint8_
         ctx->launches++;
         SWB_CUDA(cudaGetLastError());
     }
-    if (n_templates) SWB_CUDA(cudaMemcpyAsync(out, d_out, 4 * n_templates * sizeof(swb_rescued), cudaMemcpyDeviceToHost, st));
-    SWB_CUDA(cudaMemcpyAsync(n_out, d_nout, nj * 4, cudaMemcpyDeviceToHost, st));
-    if (n_cand) SWB_CUDA(cudaMemcpyAsync(n_cand, d_ncand32, nj * 4, cudaMemcpyDeviceToHost, st));
-    SWB_CUDA(cudaEventRecord(ctx->ev_stop, st));
-    SWB_CUDA(cudaStreamSynchronize(st));
+    // Counts first, then just the regions that exist: packed on the device,
+    // into pinned staging, and from there to each job's place by host threads
+    // (with all four entries per template region copied back, 20 MB per 50k
+    // mates, the call into fresh buffers took 16.4 ms instead of 13.6).
+    SWB_CUDA(cub::DeviceScan::ExclusiveSum(ctx->d_sort_tmp.p, tmp, d_nout, d_cbase, (int)nj, st));
+    unsigned long long last_off = 0;
+    if ((rc = d2h_staged(ctx, st, {DevSpan{d_nout, n_out, nj * 4}, DevSpan{d_ncand32, n_cand, n_cand ? nj * 4 : 0},
+                                   DevSpan{d_cbase + (nj - 1), &last_off, 8}})))
+        return rc;
+    const size_t total = (size_t)last_off + n_out[nj - 1];
+    if (total) {
+        if ((rc = ensure_dev(ctx, ctx->d_aux, total * sizeof(swb_rescued))) ||
+            (rc = ensure_host(ctx, ctx->h_out, total * sizeof(swb_rescued))))
+            return rc;
+        swb_rescued *d_pack = (swb_rescued *)ctx->d_aux.p;
+        const swb_rescued *packed = (const swb_rescued *)ctx->h_out.p;
+        rescue_pack_kernel<<<grid, tb, 0, st>>>(ra.jobs, nj, d_out, d_nout, d_cbase, d_pack);
+        ctx->launches++;
+        SWB_CUDA(cudaGetLastError());
+        SWB_CUDA(cudaMemcpyAsync(ctx->h_out.p, d_pack, total * sizeof(swb_rescued), cudaMemcpyDeviceToHost, st));
+        SWB_CUDA(cudaEventRecord(ctx->ev_stop, st));
+        SWB_CUDA(cudaStreamSynchronize(st));
+        const size_t nth = std::min<size_t>(std::max(1u, std::thread::hardware_concurrency()), std::max<size_t>(1, nj / 4096));
+        const size_t per = (nj + nth - 1) / nth;
+        std::vector<size_t> first(nth + 1, 0);   // packed position of each thread's first job
+        for (size_t t = 0, j = 0, at = 0; t < nth; ++t) {
+            first[t] = at;
+            for (const size_t hi = std::min(nj, (t + 1) * per); j < hi; ++j) at += n_out[j];
+        }
+        auto place = [&](size_t t) {
+            size_t at = first[t];
+            for (size_t j = std::min(nj, t * per); j < std::min(nj, (t + 1) * per); ++j) {
+                if (n_out[j]) std::memcpy(out + 4 * (size_t)jobs[j].tmpl_off, packed + at, n_out[j] * sizeof(swb_rescued));
+                at += n_out[j];
+            }
+        };
+        if (nth == 1) {
+            place(0);
+        } else {
+            std::vector<std::thread> th;
+            for (size_t t = 0; t < nth; ++t) th.emplace_back(place, t);
+            for (auto &x : th) x.join();
+        }
+    } else {
+        SWB_CUDA(cudaEventRecord(ctx->ev_stop, st));
+        SWB_CUDA(cudaStreamSynchronize(st));
+    }
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop) == cudaSuccess) ctx->last_ms = ms;
     unsigned long long c[kNumCounters] = {0};
