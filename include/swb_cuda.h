@@ -433,7 +433,10 @@ typedef struct swb_smem {
  * n_cp = (length >> 6) + 1 checkpoints, count[5] = the cumulative base
  * counts each +1 for the sentinel (count[4] = length), sentinel = the BWT
  * position of '$'.  Replaces the Metal engine's bwtCheckpointBuffer /
- * bwtCountsBuffer / bwtSentinelBuffer (MetalSWEngine.swift:88-120). */
+ * bwtCountsBuffer / bwtSentinelBuffer (MetalSWEngine.swift:88-120).  The
+ * checkpoints are kept as 32-byte blocks when length is below 2^32 - 1 and
+ * every position but the sentinel's is in exactly one bitstring, else as
+ * given; the results are the same. */
 int swb_upload_bwt(swb_ctx *ctx, const swb_bwt_checkpoint *cp, uint64_t n_cp, const int64_t count[5],
                    int64_t length, int64_t sentinel);
 

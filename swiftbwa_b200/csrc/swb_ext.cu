@@ -513,7 +513,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     const size_t set = pipe ? pipe->cap : n;
     const int slot = pipe ? pipe->slot : 0;
     if ((rc = ensure_dev(ctx, ctx->d_keys, n * 4)) || (rc = ensure_dev(ctx, ctx->d_keys2, n * 4)) ||
-        (rc = ensure_dev(ctx, ctx->d_idx, n * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, (slot + 1) * set * 6)) ||
+        (rc = ensure_dev(ctx, ctx->d_idx, n * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, (pipe ? 2 : 1) * set * 6)) ||
         (rc = ensure_dev(ctx, ctx->d_misc, (slot + 1) * kMiscBytes)))
         return rc;
     // The context's length classes at the time of the call: the keys and the
