@@ -548,9 +548,8 @@ int swb_local_align(swb_ctx *ctx, const uint8_t *query, int32_t qlen,
  * context's streams and returns, per kernel name, the launches, summed
  * device time and DP cells since the last swb_profile_reset.  The extension
  * kernels then compute every row the reference computes, so that the cells are
- * its count; without profiling they leave out rows that cannot change a
- * result (swb_ext_batch, whose cells swb_last_batch_stats reports, never
- * does), so a pass takes longer under profiling. */
+ * its count; without profiling swb_ext_batch_device leaves out rows that
+ * cannot change a result, so its pass takes longer under profiling. */
 typedef struct swb_kernel_stat {
     char     name[40];
     uint32_t launches;
@@ -570,8 +569,8 @@ int swb_int16x2_alu_peak(swb_ctx *ctx, double *lane_ops_per_s);
 /* Kernel launches issued by this context so far (for launch accounting). */
 uint64_t swb_kernel_launches(const swb_ctx *ctx);
 /* Device time (ms, CUDA events on the context's stream) of the last
- * synchronous batch call's kernels, and the DP cells it updated (for
- * swb_ext_batch those of every row the reference computes). */
+ * synchronous batch call's kernels, and the DP cells it updated (for the
+ * extension entries and chains those of every row the reference computes). */
 int swb_last_batch_stats(const swb_ctx *ctx, double *kernel_ms, uint64_t *cells);
 
 #ifdef __cplusplus

@@ -520,7 +520,8 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     // launches below use the same copy.
     const ExtBins bins = ctx->ext_bins;
     // Rows that cannot change a result are computed only where the reference's
-    // cell count is reported: by the host batch entry and under profiling.
+    // cell count is reported: by the host batch entry, the chains and the
+    // server, and under profiling.
     const bool all = all_rows || ctx->prof_on;
     const int ring_above = bins.q[bins.n - 1];
     // The rows before the first mismatch are left out in passes of more tasks

@@ -501,7 +501,7 @@ extern "C" int swb_extend_chains(swb_ctx *ctx, const swb_scoring *sc, const uint
         SWB_CUDA(cudaStreamSynchronize(st));
         if (n == 0) break;
         if ((rc = launch_ext(ctx, dsc, (const uint8_t *)ctx->d_bases.p, d_batch, n, d_res, ctx->d_counters, st,
-                             max_read, 0, nullptr, false, true)))
+                             max_read, 0, nullptr, true, true)))
             return rc;
         ++nround;
         {

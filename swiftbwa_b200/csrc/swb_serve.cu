@@ -297,7 +297,7 @@ bool launch_wave(swb_server *s, Lane &L) {
             int max_q = 0;
             for (const Piece &p : L.pieces) max_q = std::max(max_q, p.r->max_q);
             rc = launch_ext(c, s->dsc, s->d_arena, d_tasks, wn, d_out, c->d_counters, st, max_q, s->latency_cells,
-                            nullptr, false, true);
+                            nullptr, true, true);
         }
     }
     if (!rc) cudaEventRecord(L.ev_t1, st);

@@ -95,3 +95,31 @@ def test_rows_left_out(oracle_mod, si, qmax, bins):
                 assert eng.last_batch_stats()[1] == cells * rep
     finally:
         eng.close()
+
+
+def test_chains_and_server_report_every_row(oracle_mod):
+    """More tasks than the warp-per-task passes take: the cells that the chains
+    and the request loop report are the oracle's."""
+    from swiftbwa_b200 import workloads as W
+    from swiftbwa_b200.alignment import Engine
+    from swiftbwa_b200.serving import Server
+    sc = Scoring.default()
+    eng = Engine(0)
+    try:
+        ref = W.reference(W.SEED_BASE + 53, 300_000, tandem_frac=0.05)
+        wl = W.chains(ref, 91, 9000, 150, sub=0.03, indel=0.01, spurious_frac=0.3, a=sc.a)
+        eng.upload_reference(ref.pac, ref.n)
+        eng.extend_chains(sc, wl.bases, wl.seeds, wl.chains, ref.n)
+        _, _, cells = oracle_mod.extend_batch(sc, wl.bases, ref.pac, ref.n, wl.seeds, wl.chains, n_threads=8)
+        assert eng.last_batch_stats()[1] == cells
+        bases, tasks = _tasks(977, 6000, 140)
+        exp, cells = oracle_mod.ext_batch(sc, bases, tasks, n_threads=8)
+        srv = Server(eng, sc)
+        try:
+            got, _, _ = srv.wait(srv.submit(bases, tasks))
+            assert np.array_equal(got, exp)
+            assert srv.stats()["cells"] == cells
+        finally:
+            srv.stop()
+    finally:
+        eng.close()
