@@ -500,8 +500,12 @@ extern "C" int swb_extend_chains(swb_ctx *ctx, const swb_scoring *sc, const uint
         SWB_CUDA(cudaMemcpyAsync(&n, d_num, sizeof(n), cudaMemcpyDeviceToHost, st));
         SWB_CUDA(cudaStreamSynchronize(st));
         if (n == 0) break;
-        if ((rc = launch_ext(ctx, dsc, (const uint8_t *)ctx->d_bases.p, d_batch, n, d_res, ctx->d_counters, st,
-                             max_read, 0, nullptr, true, true)))
+        // A round that runs the bins has its bin sizes read back (no hint), so that
+        // the ones without tasks, most of them for short reads, are not launched (200k
+        // chains of 150 bp reads, two rounds: 5.77 -> 5.38 and 5.78 -> 4.72 ms in two runs).
+        const int hint = n > kExtWarpsMaxTasks ? -1 : max_read;
+        if ((rc = launch_ext(ctx, dsc, (const uint8_t *)ctx->d_bases.p, d_batch, n, d_res, ctx->d_counters, st, hint, 0,
+                             nullptr, true, true)))
             return rc;
         ++nround;
         {
