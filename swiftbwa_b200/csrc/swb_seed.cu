@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "swb_index.h"
 #include "swb_internal.h"
 
 namespace swb {
@@ -510,7 +511,7 @@ __global__ void __launch_bounds__(kSeedT, sizeof(U) == 4 ? 8 : 5) smem_kernel(co
 __global__ void seed_order_kernel(const uint8_t *__restrict__ bases, const uint64_t *__restrict__ read_off,
                                   const int32_t *__restrict__ read_len, uint32_t n_reads, uint32_t *__restrict__ fill,
                                   uint32_t *__restrict__ order) {
-    const uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kGrp;
+    const uint32_t r = (uint32_t)group_item(blockIdx.x, blockDim.x, threadIdx.x, kGrp);
     const int lane = threadIdx.x & 31, gl = lane & (kGrp - 1);
     unsigned long long seen = 0;
     int len = 0;
