@@ -597,9 +597,9 @@ using namespace swb;
 namespace {
 
 // Uploads the index as 32-byte blocks, the checkpoints passing through a
-// chunk buffer that is freed again (the two together never exceed the 64-byte
-// checkpoints).  compact = false: the index or the budget does not allow it,
-// nothing was kept.
+// chunk buffer that is freed again (the two together take the size of the
+// 64-byte checkpoints and up to 288 bytes).  compact = false: the index or the
+// budget does not allow it, nothing was kept.
 int upload_compact(swb_ctx *ctx, const swb_bwt_checkpoint *cp, uint64_t n_cp, int64_t length, int64_t sentinel,
                    bool &compact) {
     compact = false;
@@ -613,7 +613,6 @@ int upload_compact(swb_ctx *ctx, const swb_bwt_checkpoint *cp, uint64_t n_cp, in
         cudaGetLastError();
         return SWB_OK;
     }
-    ctx->bwt_ncp = 0;   // the index held so far is overwritten
     swb_bwt_checkpoint *d_cp = (swb_bwt_checkpoint *)tmp;
     uint32_t *d_bad = (uint32_t *)(tmp + chunk * sizeof(swb_bwt_checkpoint)), bad = 0;
     cudaError_t e = cudaMemsetAsync(d_bad, 0, 4, ctx->stream);
@@ -648,12 +647,19 @@ int swb_upload_bwt(swb_ctx *ctx, const swb_bwt_checkpoint *cp, uint64_t n_cp, co
         if (count[c] < 0 || count[c] > count[c + 1]) return set_error(SWB_ERR_INVALID_ARG, "BWT: counts must ascend");
     std::lock_guard<std::mutex> lk(ctx->mu);
     SWB_CUDA(cudaSetDevice(ctx->device));
+    // An index is accepted when the budget holds its 64-byte form, which either
+    // form may need; a refused one leaves the index held so far alone.  From
+    // here on that one is lost (its buffer is freed or overwritten), so no
+    // later failure may leave it marked as there.
+    const size_t wide = n_cp * sizeof(swb_bwt_checkpoint), others = ctx->allocated - ctx->d_bwt.cap;
+    if (n_cp > SIZE_MAX / (2 * sizeof(swb_bwt_checkpoint)) || others + ((wide + 4095) & ~(size_t)4095) > ctx->budget)
+        return set_error(SWB_ERR_OOM, "device memory budget exceeded (index of " + std::to_string(n_cp) + " checkpoints)");
+    ctx->bwt_ncp = 0;
     int rc;
     bool compact = false;
     if ((rc = upload_compact(ctx, cp, n_cp, length, sentinel, compact))) return rc;
     if (!compact) {
-        if ((rc = ensure_dev(ctx, ctx->d_bwt, n_cp * sizeof(swb_bwt_checkpoint)))) return rc;
-        ctx->bwt_ncp = 0;   // the index held so far is overwritten
+        if ((rc = ensure_dev(ctx, ctx->d_bwt, wide))) return rc;
         SWB_CUDA(cudaMemcpy(ctx->d_bwt.p, cp, n_cp * sizeof(swb_bwt_checkpoint), cudaMemcpyHostToDevice));
     }
     ctx->bwt_compact = compact;

@@ -62,3 +62,30 @@ def test_groups_equal_oracle(oracle_mod, wide, n, lmax):
     assert np.array_equal(gn, en)
     for r in range(n):
         assert np.array_equal(got[goff[r]:goff[r] + gn[r]], exp[r * cap:r * cap + en[r]]), f"read {r}"
+
+
+def test_refused_upload_keeps_the_index(oracle_mod):
+    """An index that the memory budget does not hold is refused before anything
+    is freed: the one uploaded before it still gives its SMEMs."""
+    from swiftbwa_b200 import abi
+    from swiftbwa_b200.alignment import Engine, SWBError
+    codes, idx = _index(oracle_mod, 40_000, 5)
+    bases, off, lens = _reads(codes, 7, 40, 200)
+    exp, en, _ = oracle_mod.smem_batch(idx, bases, off, lens, 15, cap=512, n_threads=8, split_len=28, split_width=10)
+    budget = 24 << 20
+    n_cp = budget * 5 // 4 // 64               # 1.25 budgets as checkpoints, 0.63 as 32-byte blocks
+    big = np.zeros(n_cp, idx.cp.dtype)
+    length = (n_cp - 1) * 64
+    eng = Engine(0, mem_budget_bytes=budget)
+    try:
+        eng.upload_bwt(idx.cp, idx.count, idx.length, idx.sentinel)
+        for _ in range(2):
+            with pytest.raises(SWBError) as ei:
+                eng.upload_bwt(big, np.array([0, 1, 2, 3, length]), length, 5)
+            assert ei.value.status == abi.SWB_ERR_OOM
+            got, gn, goff = eng.smem_batch(bases, off, lens, 15, cap_per_read=512, split_len=28)
+            assert np.array_equal(gn, en)
+            for r in range(len(lens)):
+                assert np.array_equal(got[goff[r]:goff[r] + gn[r]], exp[r * 512:r * 512 + en[r]]), f"read {r}"
+    finally:
+        eng.close()
