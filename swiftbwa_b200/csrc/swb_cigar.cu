@@ -257,7 +257,7 @@ extern "C" int swb_cigar_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_
                     r.band_bad = i;
                 ++r.nd;
                 r.raw += (size_t)t.qlen + (size_t)t.rlen;
-                r.shape.add(t.qlen, t.rlen, cost16);
+                r.shape.add(t.qlen, t.rlen, band_of(t), cost16);
             }
         });
     }
@@ -277,13 +277,7 @@ extern "C" int swb_cigar_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_
         r.dp0 = nd;
         nd += r.nd;
         raw_words += r.raw;
-        shape.n_small += r.shape.n_small;
-        shape.n_small16 += r.shape.n_small16;
-        shape.n_big += r.shape.n_big;
-        shape.small_q = std::max(shape.small_q, r.shape.small_q);
-        shape.small_t = std::max(shape.small_t, r.shape.small_t);
-        shape.big_q = std::max(shape.big_q, r.shape.big_q);
-        shape.big_t = std::max(shape.big_t, r.shape.big_t);
+        shape.add(r.shape);
     }
 
     std::lock_guard<std::mutex> lk(ctx->mu);

@@ -631,12 +631,9 @@ __global__ void __launch_bounds__(256) global_smem_kernel(GlobalArgs a, const ui
 // reference's int32 ones, sentinels included.  A lane's codes of a row are one
 // word, a row one 128-byte store; the traceback walks them with all lanes
 // holding the current row, the next rows loaded ahead.
-// Up to this many alignments: a warp holds one, so about 4,700 are in flight
-// against 44,000 with a thread each, at a third of the throughput but an eighth
-// of the time for one.  Kernel time, warp / thread per alignment, 150 bp reads:
-// band 100, 1k 134 / 674 us, 10k 821 / 717; band 5, 1k 132 / 201, 10k 820 / 254;
-// 100 bp, band 5, 8k 380 / 185; 250 bp, band 100, 1k 320 / 1252.
-constexpr size_t kNwWarpMaxTasks = 4096;
+// Which batches: nw_run_warps.  A warp holds one alignment, so about 4,700 are in
+// flight against 44,000 with a thread each, at a third of the throughput but up to
+// an eighth of the time for one.
 constexpr int kNwNone = -1500000000;   // below every sentinel-derived value
 
 template <int KC>
@@ -842,8 +839,12 @@ __global__ void __launch_bounds__(128, KC <= 5 ? 8 : 6) global_warp_kernel(Globa
 
 using NwWarpKernel = void (*)(GlobalArgs, const uint32_t *, size_t, uint32_t, uint32_t *, uint32_t *, int);
 NwWarpKernel nw_warp_kernel(int qcap) {
-    return qcap <= 128 ? global_warp_kernel<4> : qcap <= 160 ? global_warp_kernel<5>
-         : qcap <= 192 ? global_warp_kernel<6> : global_warp_kernel<8>;
+    switch (nw_warp_cols(qcap)) {
+    case 4: return global_warp_kernel<4>;
+    case 5: return global_warp_kernel<5>;
+    case 6: return global_warp_kernel<6>;
+    default: return global_warp_kernel<8>;
+    }
 }
 
 __global__ void cigar_offsets_kernel(const swb_global_task *__restrict__ tasks, size_t n,
@@ -898,7 +899,7 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     int qcap = 0, warp_grid = 0;
     const size_t n_small_of[2] = {shape.n_small - shape.n_small16, shape.n_small16};
     const int zrows = imax(shape.small_t, 1);
-    if (shape.n_small16 > 0 && shape.n_small16 <= kNwWarpMaxTasks) {
+    if (nw_run_warps(shape)) {
         // One warp per alignment: resident blocks of four, each warp with its
         // own backpointer rows.
         int occ = 0;

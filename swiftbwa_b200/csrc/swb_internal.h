@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstdlib>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -256,6 +257,7 @@ int launch_ext_plain(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
 // run in the shared-memory kernel, longer ones in the global-scratch kernel;
 // the shape gives each group's count and largest query / target.
 constexpr int kGlobalSmemMaxQ = 256;
+constexpr long long kNwRowCols = 26;   // columns that a thread's row costs besides its band's (nw_run_warps)
 // The int16-row NW kernel is exact for a task when (qlen + tlen + 2) times
 // (a + the largest single-step cost) stays below 16000 (swb_global.cu).
 __host__ __device__ inline int nw_i16_cost(int a, int b, int o_del, int e_del, int o_ins, int e_ins) {
@@ -270,10 +272,17 @@ __host__ __device__ inline bool nw_fits_i16(int qlen, int tlen, int cost) {
 struct GlobalShape {
     size_t n_small = 0, n_small16 = 0, n_big = 0;
     int small_q = 0, small_t = 0, big_q = 0, big_t = 0;
-    void add(int qlen, int tlen, int cost16) {
+    unsigned long long rows16 = 0;   // target rows of the int16-row alignments
+    long long long16 = 0;            // their largest rows * (kNwRowCols + band columns)
+    void add(int qlen, int tlen, int w, int cost16) {
         if (qlen <= kGlobalSmemMaxQ) {
             ++n_small;
-            if (nw_fits_i16(qlen, tlen, cost16)) ++n_small16;
+            if (nw_fits_i16(qlen, tlen, cost16)) {
+                ++n_small16;
+                rows16 += (unsigned long long)tlen;
+                const long long half = std::max(w, std::abs(qlen - tlen));
+                long16 = std::max(long16, tlen * (kNwRowCols + std::min<long long>(qlen, 2 * half + 1)));
+            }
             small_q = std::max(small_q, qlen);
             small_t = std::max(small_t, tlen);
         } else {
@@ -282,7 +291,33 @@ struct GlobalShape {
             big_t = std::max(big_t, tlen);
         }
     }
+    void add(const GlobalShape &o) {
+        n_small += o.n_small;
+        n_small16 += o.n_small16;
+        n_big += o.n_big;
+        small_q = std::max(small_q, o.small_q);
+        small_t = std::max(small_t, o.small_t);
+        big_q = std::max(big_q, o.big_q);
+        big_t = std::max(big_t, o.big_t);
+        rows16 += o.rows16;
+        long16 = std::max(long16, o.long16);
+    }
 };
+// The int16-row alignments run one warp each (swb_global.cu) instead of one
+// thread each while their rows together cost less than the longest alignment's
+// serial walk.  A warp's row costs by the columns a lane keeps, whatever the
+// band (about 4700 warps are in flight); a thread's row about kNwRowCols columns
+// plus those of the band.  Kernel time, warp / thread: 150 bp, band 5, 1k
+// 161 / 214 us, 1.5k 215 / 214, 4k 396 / 218; band 20, 2.5k 304 / 313, 4k
+// 396 / 314; band 100, 4k 397 / 643; 250 bp, band 5, 1k 348 / 339, band 50,
+// 3k 806 / 798; 100 bp, band 10, 3k 213 / 216.  Within a fifth of the crossing either side
+// may be chosen (100 bp, band 20, 4k: threads, 269 / 238).
+constexpr size_t kNwWarpMaxTasks = 4096;   // no more were measured with wide bands
+inline int nw_warp_cols(int qcap) { return qcap <= 128 ? 4 : qcap <= 160 ? 5 : qcap <= 192 ? 6 : 8; }
+inline bool nw_run_warps(const GlobalShape &s) {
+    return s.n_small16 > 0 && s.n_small16 <= kNwWarpMaxTasks &&
+           s.rows16 * (unsigned long long)nw_warp_cols(s.small_q) <= 220ull * (unsigned long long)s.long16;
+}
 int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
                   const swb_global_task *d_tasks, size_t n, swb_global_result *d_res,
                   uint32_t *d_cigar, unsigned long long *d_cells, cudaStream_t stream,
