@@ -241,7 +241,10 @@ int swb_local_batch(swb_ctx *ctx, const swb_scoring *sc,
 /* ------------------------------------- device-resident entry point (HBM in/out) */
 /* Same as swb_ext_batch with every pointer a device pointer on the
  * context's device, enqueued on `stream` (a cudaStream_t, NULL = the
- * context's stream); returns without synchronising. */
+ * context's stream).  Reads the batch's shape back, which synchronises
+ * `stream` once, and returns while the pass runs.  Passes and batch calls of
+ * one context share its workspace, so each waits for the ones before it,
+ * whatever their streams; use one context per stream to overlap them. */
 int swb_ext_batch_device(swb_ctx *ctx, const swb_scoring *sc,
                          const uint8_t *d_bases, const swb_ext_task *d_tasks,
                          size_t n_tasks, swb_ext_result *d_out, void *stream);

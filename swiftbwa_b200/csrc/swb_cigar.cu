@@ -284,6 +284,7 @@ extern "C" int swb_cigar_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_
     ctx->last_ms = 0;
     ctx->last_cells = 0;
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     cudaStream_t st = ctx->stream;
     const size_t n = n_tasks;
     size_t off = 0;

@@ -397,6 +397,7 @@ extern "C" int swb_extend_chains(swb_ctx *ctx, const swb_scoring *sc, const uint
 
     std::lock_guard<std::mutex> lk(ctx->mu);
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     cudaStream_t st = ctx->stream;
     const DevScoring dsc = make_dev_scoring(*sc);
     const size_t nc = n_chains, ns = std::max<size_t>(n_seeds, 1);

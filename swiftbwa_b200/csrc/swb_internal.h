@@ -130,6 +130,11 @@ struct swb_ctx {
     // host<->device copy streams and per-chunk events of the pipelined batch calls
     cudaStream_t h2d = nullptr, d2h = nullptr;
     cudaEvent_t chunk_in[swb::kMaxChunks] = {}, chunk_done[swb::kMaxChunks] = {};
+    // The pass that a device entry left running on the caller's stream.  It
+    // reads the workspace below (order, bin bounds, claim counters, rows left
+    // out, scratch), so the next call, on whatever stream, waits for it.
+    cudaEvent_t work_ev = nullptr;
+    bool work_left = false;
     size_t budget = 0;       // cap on bytes the context allocates on the device
     size_t allocated = 0;    // bytes currently allocated
     std::mutex mu;
@@ -202,6 +207,11 @@ void par_copy(void *dst, const void *src, size_t bytes);
 // True when p lies in page-locked host memory (cudaHostAlloc or registered).
 bool is_pinned(const void *p);
 int d2h_staged(swb_ctx *ctx, cudaStream_t st, std::initializer_list<DevSpan> parts, cudaEvent_t after_copies = nullptr);
+
+// The workspace passes from call to call: work_acquire makes `s` wait for the
+// pass that a device entry left running, work_leave marks one on `s`.
+int work_acquire(swb_ctx *ctx, cudaStream_t s);
+void work_leave(swb_ctx *ctx, cudaStream_t s);
 
 // Grow-only allocation against the context budget.
 int ensure_dev(swb_ctx *ctx, DevBuf &b, size_t bytes);

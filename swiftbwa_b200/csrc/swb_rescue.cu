@@ -250,6 +250,7 @@ extern "C" int swb_mate_rescue(swb_ctx *ctx, const swb_scoring *sc, const uint8_
 
     std::lock_guard<std::mutex> lk(ctx->mu);
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     cudaStream_t st = ctx->stream;
     const size_t nj = n_jobs, nt = std::max<size_t>(n_templates, 1), nmr = std::max<size_t>(n_mate_regions, 1);
     const uint64_t rc_base = al256(std::max<size_t>(n_bases, 1));

@@ -36,6 +36,17 @@ int check_cuda(cudaError_t e, const char *what) {
     return set_error(SWB_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+int work_acquire(swb_ctx *ctx, cudaStream_t s) {
+    if (ctx->work_left) SWB_CUDA(cudaStreamWaitEvent(s, ctx->work_ev, 0));
+    return SWB_OK;
+}
+
+void work_leave(swb_ctx *ctx, cudaStream_t s) {
+    // (without the event, the wait the call would have left to the next one)
+    if (cudaEventRecord(ctx->work_ev, s) == cudaSuccess) ctx->work_left = true;
+    else cudaStreamSynchronize(s);
+}
+
 int ensure_dev(swb_ctx *ctx, DevBuf &b, size_t bytes) {
     if (bytes <= b.cap) return SWB_OK;
     size_t want = std::max(bytes, b.cap + b.cap / 2);
@@ -49,6 +60,7 @@ int ensure_dev(swb_ctx *ctx, DevBuf &b, size_t bytes) {
     }
     if (b.p) {
         cudaStreamSynchronize(ctx->stream);
+        if (ctx->work_left) cudaEventSynchronize(ctx->work_ev);
         cudaFree(b.p);
         ctx->allocated -= b.cap;
         b.p = nullptr;
@@ -432,6 +444,7 @@ int swb_init(int device, size_t mem_budget_bytes, swb_ctx **out) {
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->join_ev[k], cudaEventDisableTiming);
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->work_ev, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking);
     for (int k = 0; k < kMaxChunks && e == cudaSuccess; ++k) {
@@ -452,6 +465,7 @@ void swb_destroy(swb_ctx *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    if (ctx->work_left) cudaEventSynchronize(ctx->work_ev);
     DevBuf *bufs[] = {&ctx->d_bases, &ctx->d_tasks, &ctx->d_out, &ctx->d_keys, &ctx->d_keys2, &ctx->d_idx,
                       &ctx->d_idx2, &ctx->d_sort_tmp, &ctx->d_misc, &ctx->d_scratch, &ctx->d_cigar, &ctx->d_aux, &ctx->d_chain,
                       &ctx->d_bwt, &ctx->d_seed};
@@ -472,6 +486,7 @@ void swb_destroy(swb_ctx *ctx) {
         if (ctx->join_ev[k]) cudaEventDestroy(ctx->join_ev[k]);
     }
     if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
+    if (ctx->work_ev) cudaEventDestroy(ctx->work_ev);
     for (cudaStream_t st : {ctx->h2d, ctx->d2h})
         if (st) {
             cudaStreamSynchronize(st);
@@ -492,6 +507,7 @@ int swb_upload_reference(swb_ctx *ctx, const uint8_t *pac, uint64_t n_bases) {
     const size_t bytes = (size_t)((n_bases + 3) / 4);
     if (ctx->d_pac) {
         cudaStreamSynchronize(ctx->stream);
+        if (ctx->work_left) cudaEventSynchronize(ctx->work_ev);
         cudaFree(ctx->d_pac);
         ctx->allocated -= ctx->pac_bytes;
         ctx->d_pac = nullptr;
@@ -519,6 +535,7 @@ int swb_ext_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, siz
     ctx->last_cells = 0;
     if (n_tasks == 0) return SWB_OK;
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     const DevScoring dsc = make_dev_scoring(*sc);
 
     // Large batches (8M tasks and up): chunks that grow by half from 1/32 of
@@ -704,6 +721,7 @@ int swb_tune_ext_bins(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases,
     const std::vector<ExtBins> cand = ext_bin_candidates(tasks, n_tasks, dsc);
     std::lock_guard<std::mutex> lk(ctx->mu);
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     const ExtBins keep = ctx->ext_bins;
     // Any early return (a failed CUDA call) puts the caller's classes back.
     struct Restore {
@@ -773,7 +791,10 @@ int swb_ext_batch_device(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *d_b
     if (n_tasks == 0) return SWB_OK;
     SWB_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    return launch_ext(ctx, make_dev_scoring(*sc), d_bases, d_tasks, n_tasks, d_out, ctx->d_counters, s, -1);
+    if ((rc = work_acquire(ctx, s))) return rc;
+    rc = launch_ext(ctx, make_dev_scoring(*sc), d_bases, d_tasks, n_tasks, d_out, ctx->d_counters, s, -1);
+    work_leave(ctx, s);
+    return rc;
 }
 
 int swb_ext_batch_plain_device(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *d_bases,
@@ -785,7 +806,10 @@ int swb_ext_batch_plain_device(swb_ctx *ctx, const swb_scoring *sc, const uint8_
     if (n_tasks == 0) return SWB_OK;
     SWB_CUDA(cudaSetDevice(ctx->device));
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    return launch_ext_plain(ctx, make_dev_scoring(*sc), d_bases, d_tasks, n_tasks, d_out, ctx->d_counters, s);
+    if ((rc = work_acquire(ctx, s))) return rc;
+    rc = launch_ext_plain(ctx, make_dev_scoring(*sc), d_bases, d_tasks, n_tasks, d_out, ctx->d_counters, s);
+    work_leave(ctx, s);
+    return rc;
 }
 
 int swb_global_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, size_t n_bases,
@@ -813,6 +837,7 @@ int swb_global_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, 
     }
     if (need > cigar_cap) return set_error(SWB_ERR_INVALID_ARG, "cigar_cap below sum of (qlen + tlen)");
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     const DevScoring dsc = make_dev_scoring(*sc);
     void *d_b = nullptr, *d_t = nullptr;
     if ((rc = stage_in(ctx, {Part{bases, n_bases, &d_b}, Part{tasks, n_tasks * sizeof(swb_global_task), &d_t}}))) return rc;
@@ -848,6 +873,7 @@ int swb_local_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, s
     int max_q = 0, max_t = 0;
     if ((rc = validate_spans(ctx, tasks, n_tasks, n_bases, &max_q, &max_t))) return rc;
     SWB_CUDA(cudaSetDevice(ctx->device));
+    if ((rc = work_acquire(ctx, ctx->stream))) return rc;
     const DevScoring dsc = make_dev_scoring(*sc);
     void *d_b = nullptr, *d_t = nullptr;
     if ((rc = stage_in(ctx, {Part{bases, n_bases, &d_b}, Part{tasks, n_tasks * sizeof(swb_local_task), &d_t}}))) return rc;

@@ -702,7 +702,7 @@ int swb_smem_batch(swb_ctx *ctx, const uint8_t *bases, size_t n_bases, const uin
     SWB_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, (unsigned long long *)nullptr,
                                            (unsigned long long *)nullptr, (int)n_reads, ctx->stream));
     int rc;
-    if ((rc = ensure_dev(ctx, ctx->d_idx, n_reads * 4))) return rc;
+    if ((rc = work_acquire(ctx, st)) || (rc = ensure_dev(ctx, ctx->d_idx, n_reads * 4))) return rc;
     if ((rc = ensure_dev(ctx, ctx->d_bases, b_bytes + o_bytes + l_bytes + 256)) ||
         (rc = ensure_dev(ctx, ctx->d_out, out_bytes + n_bytes + 2 * off_bytes + al(scan_bytes) + 256)))
         return rc;
