@@ -56,7 +56,8 @@ namespace {
 // int32 rows (one warp per extension, or global scratch above kWarpMaxQ).
 constexpr int kFastT = 32;                // threads per block in the shared-memory kernels
 // Per pass: bin bounds (up to 32 words), the int32 bin's longest query at
-// byte 256, the bins' claim counters from byte 320.
+// byte 256, a zero at byte 264 (passes without rows left out), the bins' claim
+// counters from byte 320.
 constexpr size_t kMiscBytes = 512;
 constexpr int kBigT = 64;
 constexpr size_t kSmemPerSm = 227 * 1024;
@@ -101,10 +102,11 @@ __device__ __forceinline__ int ext_bin(const swb_ext_task &t, const DevScoring &
 // largest first: the lanes of a warp run similar numbers of rows of similar
 // width, and within a bin the tasks with the most work start first and overlap
 // the rest instead of finishing the bin alone.  The rows are those after the
-// ones left out at the start (skip[i], ext_skip_rows), up to the target's end,
-// or with all = 0 about the query's length, where most tasks stop.
+// ones left out at the start (skip[i], ext_skip_rows; none if skip is NULL), up
+// to the target's end, or with all = 0 about the query's length, where most
+// tasks stop.
 __global__ void ext_keys_kernel(const swb_ext_task *__restrict__ tasks, size_t n, DevScoring sc, int pair_ok,
-                                uint32_t warp_cells, ExtBins bins, int ring_above, int all, int skip_rows,
+                                uint32_t warp_cells, ExtBins bins, int ring_above, int all,
                                 const uint8_t *__restrict__ bases, const uint8_t *__restrict__ pac,
                                 uint32_t *__restrict__ keys, uint32_t *__restrict__ idx, uint16_t *__restrict__ skip,
                                 int *__restrict__ big_max_q) {
@@ -114,14 +116,14 @@ __global__ void ext_keys_kernel(const swb_ext_task *__restrict__ tasks, size_t n
     int len = task_row_len(t, sc, ring_above), s = 0;
     int b = ext_bin(t, sc, pair_ok != 0, warp_cells, bins, len);
     const bool pair = b < 2 * bins.n && t.qlen > 0 && t.tlen > 0;
-    if (pair && skip_rows && len == t.qlen) {
+    if (pair && skip && len == t.qlen) {
         s = ext_skip_rows(t, sc, bases, pac);
         if (s > 0) {   // the columns left: maybe a smaller class
             len -= ext_start_col(sc, ext_band_w(t.qlen, t.w, t.end_bonus, sc), t.h0, s);
             b = ext_bin(t, sc, true, 0, bins, len);
         }
     }
-    skip[i] = (uint16_t)s;
+    if (skip) skip[i] = (uint16_t)s;
     const uint32_t q = (uint32_t)min(max(pair ? len : t.qlen, 0), 2047);
     const int rows = (pair && !all ? min(t.tlen, t.qlen + kTailRows) : t.tlen) - s;
     const uint32_t wide = (uint32_t)min(max(min(t.w, t.qlen), 0) >> 4, 15);
@@ -182,7 +184,7 @@ __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qca
         if (pos < hi) {
             swb_ext_result r;
             const bool sym = a.sc.o_del + a.sc.e_del == a.sc.o_ins + a.sc.e_ins;
-            const int skip = a.skip[ti];
+            const int skip = a.skip[ti & a.skip_mask];
             auto run = [&](auto symc, auto ringc) {
                 constexpr bool kSym = decltype(symc)::value, kRing = decltype(ringc)::value;
                 if constexpr (U8) ext_pair_one<T, kSym, false, kRing, ALL, AHEAD>(a, tk, skip, he16, qc, r, cells);
@@ -420,6 +422,14 @@ int fast_occupancy(bool u8, bool all, bool ahead, int qcap) {
     return occ;
 }
 
+// The rows before the first mismatch are left out in passes of more tasks
+// than the GPU holds lanes of these kernels (about 20 one-warp blocks per
+// SM).  A smaller pass lasts as long as its longest task, and lanes that
+// start at different rows take longer over each (uneven tasks, rows left out
+// / kept: 8k 1455 / 1242 us, 64k 1436 / 1330, 256k 2169 / 2310, 1M 6679 / 7731;
+// 150 bp reads: 16k 532 / 533, 64k 684 / 710, 1M 2232 / 2998).
+bool leaves_first_rows(const swb_ctx *ctx, size_t n) { return n > (size_t)ctx->sm_count * 20 * kFastT; }
+
 // n: the pass's tasks; in_bin: at least the bin's.
 int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, size_t in_bin,
                 cudaStream_t s) {
@@ -443,17 +453,25 @@ int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int 
 
 }  // namespace
 
-int ext_reserve(swb_ctx *ctx, size_t cap) {
-    if (cap > 0x7FFFFFF0ull) return set_error(SWB_ERR_TOO_LARGE, "more than 2^31-16 tasks in one batch");
+// The binned pass's workspace: `sets` orders of `cap` tasks.  The rows left out
+// (2 bytes a task behind the orders) are taken only where the budget allows it
+// besides the rest: without them every first row is computed.
+static int ext_workspace(swb_ctx *ctx, size_t cap, int sets) {
     int rc;
     size_t tmp_bytes = 0;
     SWB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (uint32_t *)nullptr, (uint32_t *)nullptr,
                                              (uint32_t *)nullptr, (uint32_t *)nullptr, (int)cap, 0, 32, ctx->stream));
     if ((rc = ensure_dev(ctx, ctx->d_keys, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_keys2, cap * 4)) ||
-        (rc = ensure_dev(ctx, ctx->d_idx, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, 2 * cap * 6)) ||
-        (rc = ensure_dev(ctx, ctx->d_misc, 2 * kMiscBytes)) || (rc = ensure_dev(ctx, ctx->d_sort_tmp, tmp_bytes)))
+        (rc = ensure_dev(ctx, ctx->d_idx, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_misc, sets * kMiscBytes)) ||
+        (rc = ensure_dev(ctx, ctx->d_sort_tmp, tmp_bytes)))
         return rc;
-    return SWB_OK;
+    if (leaves_first_rows(ctx, cap) && ensure_dev(ctx, ctx->d_idx2, sets * cap * 6) == SWB_OK) return SWB_OK;
+    return ensure_dev(ctx, ctx->d_idx2, sets * cap * 4);
+}
+
+int ext_reserve(swb_ctx *ctx, size_t cap) {
+    if (cap > 0x7FFFFFF0ull) return set_error(SWB_ERR_TOO_LARGE, "more than 2^31-16 tasks in one batch");
+    return ext_workspace(ctx, cap, 2);
 }
 
 // Small batches: one warp per extension, one launch (two with queries above
@@ -512,10 +530,8 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     // claim counters (misc) are read by the bins, one set per pipelined slot.
     const size_t set = pipe ? pipe->cap : n;
     const int slot = pipe ? pipe->slot : 0;
-    if ((rc = ensure_dev(ctx, ctx->d_keys, n * 4)) || (rc = ensure_dev(ctx, ctx->d_keys2, n * 4)) ||
-        (rc = ensure_dev(ctx, ctx->d_idx, n * 4)) || (rc = ensure_dev(ctx, ctx->d_idx2, (pipe ? 2 : 1) * set * 6)) ||
-        (rc = ensure_dev(ctx, ctx->d_misc, (slot + 1) * kMiscBytes)))
-        return rc;
+    const size_t orders = (pipe ? 2 : 1) * set;
+    if (!pipe && (rc = ext_workspace(ctx, n, 1))) return rc;   // (a pipelined pass has its own from ext_reserve)
     // The context's length classes at the time of the call: the keys and the
     // launches below use the same copy.
     const ExtBins bins = ctx->ext_bins;
@@ -524,21 +540,17 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     // server, and under profiling.
     const bool all = all_rows || ctx->prof_on;
     const int ring_above = bins.q[bins.n - 1];
-    // The rows before the first mismatch are left out in passes of more tasks
-    // than the GPU holds lanes of these kernels (about 20 one-warp blocks per
-    // SM).  A smaller pass lasts as long as its longest task, and lanes that
-    // start at different rows take longer over each (uneven tasks, rows left out
-    // / kept: 8k 1455 / 1242 us, 64k 1436 / 1330, 256k 2169 / 2310, 1M 6679 / 7731;
-    // 150 bp reads: 16k 532 / 533, 64k 684 / 710, 1M 2232 / 2998).
-    const int skip_rows = n > (size_t)ctx->sm_count * 20 * kFastT;
     const int nbins = 2 * bins.n + 1, big = 2 * bins.n;
     uint32_t *keys = (uint32_t *)ctx->d_keys.p, *keys2 = (uint32_t *)ctx->d_keys2.p;
     uint32_t *idx = (uint32_t *)ctx->d_idx.p, *idx2 = (uint32_t *)ctx->d_idx2.p + (size_t)slot * set;
-    // The rows each task leaves out, behind the sets' orders.
-    uint16_t *skip = (uint16_t *)((uint32_t *)ctx->d_idx2.p + (pipe ? 2 : 1) * set) + (size_t)slot * set;
+    // The rows each task leaves out, behind the sets' orders (ext_workspace).
+    uint16_t *skip = leaves_first_rows(ctx, n) && ctx->d_idx2.cap >= orders * 6
+                         ? (uint16_t *)((uint32_t *)ctx->d_idx2.p + orders) + (size_t)slot * set
+                         : nullptr;
     char *misc = (char *)ctx->d_misc.p + slot * kMiscBytes;
     uint32_t *bin_start = (uint32_t *)misc;                   // nbins + 1 words
     int *big_max_q = (int *)(misc + 256);
+    const uint16_t *no_skip = (const uint16_t *)(misc + 264);   // a zero
     uint32_t *claim = (uint32_t *)(misc + 320);               // nbins claim counters
     SWB_CUDA(cudaMemsetAsync(misc + 256, 0, kMiscBytes - 256, s));   // big_max_q and the counters
     const unsigned tb = 256;
@@ -547,14 +559,13 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         // Two target rows per pass on 16-bit lanes: the gap costs must fit a lane.
         const int pair_ok = sc.o_del + sc.e_del <= 32767 && sc.o_ins + sc.e_ins <= 32767;
         ext_keys_kernel<<<(unsigned)((n + tb - 1) / tb), tb, 0, s>>>(d_tasks, n, sc, pair_ok, warp_cells, bins,
-                                                                       ring_above, all, skip_rows, d_bases, ctx->d_pac,
+                                                                       ring_above, all, d_bases, ctx->d_pac,
                                                                        keys, idx, skip, big_max_q);
     }
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
     size_t tmp_bytes = 0;
     SWB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, idx, idx2, (int)n, 0, 32, s));
-    if ((rc = ensure_dev(ctx, ctx->d_sort_tmp, tmp_bytes))) return rc;
     {
         ProfScope ps(ctx, s, "cub_radix_sort", -1);
         SWB_CUDA(cub::DeviceRadixSort::SortPairs(ctx->d_sort_tmp.p, tmp_bytes, keys, keys2, idx, idx2,
@@ -600,7 +611,8 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
 
     // Fork: every bin runs on its own stream after the sort, then joins back
     // (into the pipeline's join stream for pipelined passes).
-    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, d_cells, claim, ring_above, skip};
+    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, d_cells, claim, ring_above, skip ? skip : no_skip,
+              skip ? 0xFFFFFFFFu : 0u};
     const cudaStream_t js = pipe ? pipe->join : s;
     ProfScope pass(ctx, s, pipe ? nullptr : "ext_pass", -1);   // fork to join, on the launching stream
     SWB_CUDA(cudaEventRecord(ctx->fork_ev, s));
