@@ -342,17 +342,20 @@ extern "C" int swb_mate_rescue(swb_ctx *ctx, const swb_scoring *sc, const uint8_
     // Counts first, then just the regions that exist: packed on the device,
     // into pinned staging, and from there to each job's place by host threads
     // (with all four entries per template region copied back, 20 MB per 50k
-    // mates, the call into fresh buffers took 16.4 ms instead of 13.6).
+    // mates, the call into fresh buffers took 16.4 ms instead of 13.6).  Where
+    // the memory budget has no room for the packed copy, all entries cross.
     SWB_CUDA(cub::DeviceScan::ExclusiveSum(ctx->d_sort_tmp.p, tmp, d_nout, d_cbase, (int)nj, st));
     unsigned long long last_off = 0;
     if ((rc = d2h_staged(ctx, st, {DevSpan{d_nout, n_out, nj * 4}, DevSpan{d_ncand32, n_cand, n_cand ? nj * 4 : 0},
                                    DevSpan{d_cbase + (nj - 1), &last_off, 8}})))
         return rc;
     const size_t total = (size_t)last_off + n_out[nj - 1];
-    if (total) {
-        if ((rc = ensure_dev(ctx, ctx->d_aux, total * sizeof(swb_rescued))) ||
-            (rc = ensure_host(ctx, ctx->h_out, total * sizeof(swb_rescued))))
-            return rc;
+    if (total && (ensure_dev(ctx, ctx->d_aux, total * sizeof(swb_rescued)) ||
+                  ensure_host(ctx, ctx->h_out, total * sizeof(swb_rescued)))) {
+        SWB_CUDA(cudaMemcpyAsync(out, d_out, 4 * n_templates * sizeof(swb_rescued), cudaMemcpyDeviceToHost, st));
+        SWB_CUDA(cudaEventRecord(ctx->ev_stop, st));
+        SWB_CUDA(cudaStreamSynchronize(st));
+    } else if (total) {
         swb_rescued *d_pack = (swb_rescued *)ctx->d_aux.p;
         const swb_rescued *packed = (const swb_rescued *)ctx->h_out.p;
         rescue_pack_kernel<<<grid, tb, 0, st>>>(ra.jobs, nj, d_out, d_nout, d_cbase, d_pack);

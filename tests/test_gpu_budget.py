@@ -31,3 +31,50 @@ def test_extension_pass_without_room_for_rows_left_out():
             eng.close()
     assert np.array_equal(got[25 * n], got[0])
     assert isinstance(got[23 * n], int) and got[23 * n] == abi.SWB_ERR_OOM
+
+
+def _least_budget(call, lo, hi, step=1 << 16):
+    """The smallest budget (to `step`) with which call(budget) is not refused."""
+    while hi - lo > step:
+        mid = (lo + hi) // 2
+        if call(mid) is None:
+            lo = mid
+        else:
+            hi = mid
+    return hi
+
+
+def test_rescue_without_room_for_the_packed_regions(oracle_mod):
+    """A call whose mates find nothing needs everything but the packed copy of
+    the regions: with the least budget for it, the mates that find regions get
+    them too."""
+    from swiftbwa_b200 import workloads as W
+    from swiftbwa_b200.alignment import Engine, SWBError
+    ref = W.reference(W.SEED_BASE + 63, 500_000)
+    wl = W.rescue_jobs(ref, 64, 12_000, 100, n_contigs=3)
+    args = (wl.bases, wl.jobs, wl.templates, wl.mate_regions, wl.stats, wl.primary, wl.contig_offsets,
+            wl.contig_lengths, wl.ref.n)
+    sc, none = Scoring.default(), Scoring.default(min_seed_len=1000)
+
+    def call(budget, scoring):
+        eng = Engine(0, mem_budget_bytes=budget)
+        try:
+            eng.upload_reference(ref.pac, ref.n)
+            return eng.mate_rescue(scoring, *args)
+        except SWBError as e:
+            assert e.status == abi.SWB_ERR_OOM
+            return None
+        finally:
+            eng.close()
+
+    least = _least_budget(lambda b: call(b, none), 1 << 20, 1 << 30)
+    assert int(call(least, none)[1].sum()) == 0
+    got = call(least, sc)
+    assert got is not None, "refused for want of room for the packed regions"
+    exp, en, _, _ = oracle_mod.mate_rescue_batch(sc, wl.bases, wl.ref.pac, wl.ref.n, wl.jobs, wl.templates,
+                                                 wl.mate_regions, wl.stats, wl.primary, wl.contig_offsets,
+                                                 wl.contig_lengths, n_threads=8)
+    assert np.array_equal(got[1], en) and int(en.sum()) * abi.RESCUED_DTYPE.itemsize > 1 << 18
+    for j, job in enumerate(wl.jobs):
+        o, k = 4 * int(job["tmpl_off"]), int(en[j])
+        assert np.array_equal(got[0][o:o + k], exp[o:o + k]), j
