@@ -899,15 +899,18 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     int qcap = 0, warp_grid = 0;
     const size_t n_small_of[2] = {shape.n_small - shape.n_small16, shape.n_small16};
     const int zrows = imax(shape.small_t, 1);
+    const size_t big_q = (size_t)imax(shape.big_q, 1), big_t = (size_t)imax(shape.big_t, 1);
+    const size_t big_slot = (big_q + 1) * 8 + big_q + big_t + big_t * big_q;   // a longer query's rows and backpointers
     if (nw_run_warps(shape)) {
         // One warp per alignment: resident blocks of four, each warp with its
-        // own backpointer rows.
+        // own backpointer rows.  They are longer than a thread's, so with long
+        // queries in the batch they leave the scratch that those need at least.
         int occ = 0;
         SWB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, nw_warp_kernel(imax(shape.small_q, 1)), 128, 0));
         warp_grid = (int)std::min<size_t>((size_t)ctx->sm_count * imax(occ, 1), (shape.n_small16 + 3) / 4);
-        while (warp_grid > 1 && (size_t)warp_grid * 4 * zrows * 128 > avail0) warp_grid /= 2;
+        const size_t big = shape.n_big ? kGT * big_slot : 0, room = avail0 > big ? avail0 - big : 0;
         z_bytes = ((size_t)warp_grid * 4 * zrows * 128 + 1023) & ~(size_t)1023;
-        if (z_bytes > avail0) warp_grid = 0, z_bytes = 0;
+        if (z_bytes > room) warp_grid = 0, z_bytes = 0;
     }
     if (shape.n_small > 0) {
         qcap = imax(shape.small_q, 1);
@@ -947,19 +950,17 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     Scratch s{};
     size_t big_bytes = 0, grid_b = 0;
     if (shape.n_big > 0) {
-        const int qmax = imax(shape.big_q, 1), tmax = imax(shape.big_t, 1);
-        const size_t per_slot = (size_t)(qmax + 1) * 8 + (size_t)qmax + (size_t)tmax + (size_t)tmax * qmax;
         size_t nslots = std::min((size_t)ctx->sm_count * 8 * kGT, ((shape.n_big + kGT - 1) / kGT) * kGT);
         const size_t avail = avail0 > z_bytes ? avail0 - z_bytes : 0;
-        while (nslots > kGT && nslots * per_slot > avail) nslots /= 2;
+        while (nslots > kGT && nslots * big_slot > avail) nslots /= 2;
         nslots = (nslots / kGT) * kGT;
-        if (nslots == 0 || nslots * per_slot > avail)
+        if (nslots == 0 || nslots * big_slot > avail)
             return set_error(SWB_ERR_OOM, "global alignment scratch does not fit the memory budget");
         grid_b = nslots / kGT;
-        big_bytes = nslots * per_slot + 1024;
+        big_bytes = nslots * big_slot + 1024;
         s.nslots = nslots;
-        s.qmax = qmax;
-        s.tmax = tmax;
+        s.qmax = (int)big_q;
+        s.tmax = (int)big_t;
     }
     if ((rc = ensure_dev(ctx, ctx->d_scratch, z_bytes + big_bytes + 256))) return rc;
     uint32_t *claim = (uint32_t *)((char *)ctx->d_scratch.p + z_bytes + big_bytes);   // one counter per row width

@@ -78,3 +78,36 @@ def test_rescue_without_room_for_the_packed_regions(oracle_mod):
     for j, job in enumerate(wl.jobs):
         o, k = 4 * int(job["tmpl_off"]), int(en[j])
         assert np.array_equal(got[0][o:o + k], exp[o:o + k]), j
+
+
+def test_global_batch_whose_warps_would_take_the_long_queries_scratch(oracle_mod):
+    """3000 short alignments and a long one (64 slots of 4 MB): the short ones'
+    backpointers take 15 MB with a warp each and 2 MB with a thread each, and the
+    budget leaves 8 MB."""
+    from swiftbwa_b200.alignment import Engine
+    rng = np.random.default_rng(65)
+    L = 2000
+    rows = [(0, L, L, L, 50, 0, 0, 0)]
+    q = rng.integers(0, 4, L).astype(np.uint8)
+    t = q.copy()
+    t[rng.random(L) < 0.03] = 2
+    chunks, off = [q, t], 2 * L
+    for _ in range(3000):
+        x = rng.integers(0, 4, 32).astype(np.uint8)
+        chunks += [x, gen.mutate(rng, np.resize(x, 40), sub=0.03, indel=0.0)]
+        rows.append((off, off + 32, 32, len(chunks[-1]), 30, 0, 0, 0))
+        off += 32 + len(chunks[-1])
+    bases, tasks = np.concatenate(chunks), np.array(rows, dtype=abi.GLOBAL_TASK_DTYPE)
+    sc = Scoring.default()
+    eres, ecig, _ = oracle_mod.global_batch(sc, bases, tasks, n_threads=8)
+    least = 64 * ((L + 1) * 8 + 2 * L + L * L)
+    eng = Engine(0, mem_budget_bytes=2 * (least + (8 << 20)))
+    try:
+        res, cig = eng.global_batch(sc, bases, tasks)
+    finally:
+        eng.close()
+    for f in ("score", "n_cigar", "w_used", "attempts"):
+        assert np.array_equal(res[f], eres[f]), f
+    for k in range(len(tasks)):
+        o, n, eo = int(res["cigar_off"][k]), int(res["n_cigar"][k]), int(eres["cigar_off"][k])
+        assert np.array_equal(cig[o:o + n], ecig[eo:eo + n]), k
