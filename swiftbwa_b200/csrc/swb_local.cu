@@ -98,7 +98,7 @@ struct PassOut {
 // to the striped shortcuts), so the reverse maximum is the forward score.
 // (WRAP: the arithmetic may lose alignments, so only a*qLen bounds it.)
 __device__ __forceinline__ int rev_cap(const DevScoring &sc, bool wrap, int qLen, int fwd_score) {
-    const int gOEE = sc.o_ins + 2 * sc.e_ins;
+    const int gOEE = ((sc.o_ins + sc.e_ins) & 0xFF) + (sc.e_ins & 0xFF);   // the bytes that striped_pass uses
     return !wrap && fwd_score >= sc.a * (qLen - 1) - gOEE ? fwd_score : sc.a * qLen;
 }
 

@@ -99,3 +99,19 @@ def test_rescue_primary_failed_and_errors(engine, oracle_mod):
         engine.mate_rescue(Scoring.default(), wl.bases, bad, wl.templates, wl.mate_regions, wl.stats, 1,
                            wl.contig_offsets, wl.contig_lengths, ref.n)
     assert ei.value.status == abi.SWB_ERR_INVALID_ARG
+
+
+def test_rescue_gap_costs_beyond_a_byte(engine, oracle_mod):
+    """Gap costs that the byte arithmetic cuts to small ones (257 -> 1): mates
+    with many indels in tandem repeats, whose reverse pass may pass the forward
+    score and then begins elsewhere."""
+    import gen
+    from swiftbwa_b200 import workloads as W
+    ref = W.reference(W.SEED_BASE + 86, 300_000, tandem_frac=0.5)
+    wl = W.rescue_jobs(ref, 87, 6000, 120, n_contigs=2, no_hit_frac=0.0, hit_frac=0.0)
+    rng = np.random.default_rng(88)
+    bases = wl.bases.copy()
+    for m in bases.reshape(-1, 120):
+        m[:] = np.resize(gen.mutate(rng, m.copy(), sub=0.03, indel=0.06), 120)
+    wl.bases = bases
+    assert _compare(engine, oracle_mod, Scoring.default(o_ins=0, e_ins=257, o_del=0, e_del=257), wl) > 0
