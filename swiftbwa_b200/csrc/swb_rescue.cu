@@ -22,6 +22,7 @@
 #include <cub/device/device_scan.cuh>
 
 #include "swb_device.cuh"
+#include "swb_host.h"
 #include "swb_internal.h"
 
 namespace swb {
@@ -378,13 +379,7 @@ extern "C" int swb_mate_rescue(swb_ctx *ctx, const swb_scoring *sc, const uint8_
                 at += n_out[j];
             }
         };
-        if (nth == 1) {
-            place(0);
-        } else {
-            std::vector<std::thread> th;
-            for (size_t t = 0; t < nth; ++t) th.emplace_back(place, t);
-            for (auto &x : th) x.join();
-        }
+        run_parts(nth, place);
     } else {
         SWB_CUDA(cudaEventRecord(ctx->ev_stop, st));
         SWB_CUDA(cudaStreamSynchronize(st));
