@@ -61,6 +61,10 @@ constexpr int kFastT = 32;                // threads per block in the shared-mem
 constexpr size_t kMiscBytes = 512;
 constexpr int kBigT = 64;
 constexpr size_t kSmemPerSm = 227 * 1024;
+// Shared memory that the blocks of the kernels with rows per warp use at most.
+// The kernel's limit is always set to this: it belongs to the process, so a
+// limit of each call's own could be lowered by another thread's before the launch.
+constexpr size_t kWarpSmem = 200 * 1024;
 constexpr size_t kAheadBlocks = 13;
 // Rows past the query's length that a task is taken to run when it may stop
 // early (sort key only).
@@ -491,9 +495,8 @@ int launch_ext_warps(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     }
     if (max_q > kExtWarpsMaxQ) {
         const size_t stride = ((size_t)(max_q + 1) * 8 + (size_t)max_q + 15) & ~(size_t)15;
-        const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / stride));
-        SWB_CUDA(cudaFuncSetAttribute(ext_warps_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(warps * stride)));
+        const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, kWarpSmem / stride));
+        SWB_CUDA(cudaFuncSetAttribute(ext_warps_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWarpSmem));
         ProfScope ps(ctx, s, "ext_warps_long", kCntExtBin0 + 1);
         ext_warps_long_kernel<<<(unsigned)std::min<size_t>((n + warps - 1) / warps, (size_t)ctx->sm_count * 16), warps * 32,
                                 warps * stride, s>>>(a, (uint32_t)n, kExtWarpsMaxQ + 1, max_q);
@@ -601,9 +604,8 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     const size_t wstride = ((size_t)(wq + 1) * 8 + (size_t)wq + 15) & ~(size_t)15;
     int wwarps = 0, wblocks = 0;
     if (max_q > 0) {
-        wwarps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / wstride));
-        SWB_CUDA(cudaFuncSetAttribute(ext_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(wwarps * wstride)));
+        wwarps = (int)std::max<size_t>(1, std::min<size_t>(8, kWarpSmem / wstride));
+        SWB_CUDA(cudaFuncSetAttribute(ext_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWarpSmem));
         SWB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wblocks, ext_warp_kernel, wwarps * 32,
                                                                wwarps * wstride));
         wblocks = imax(wblocks, 1) * ctx->sm_count;
@@ -714,10 +716,9 @@ int launch_ext_plain(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     if (sh.big_max_q > 0) {
         const int wq = imin(sh.big_max_q, kWarpMaxQ);
         const size_t wstride = ((size_t)(wq + 1) * 8 + (size_t)wq + 15) & ~(size_t)15;
-        const int wwarps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)(200 * 1024) / wstride));
+        const int wwarps = (int)std::max<size_t>(1, std::min<size_t>(8, kWarpSmem / wstride));
         int wblocks = 0;
-        SWB_CUDA(cudaFuncSetAttribute(ext_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(wwarps * wstride)));
+        SWB_CUDA(cudaFuncSetAttribute(ext_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWarpSmem));
         SWB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&wblocks, ext_warp_kernel, wwarps * 32,
                                                                wwarps * wstride));
         wblocks = imax(wblocks, 1) * ctx->sm_count;

@@ -940,8 +940,9 @@ int launch_global(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
             while (c.grid > 1 && (size_t)c.grid * T * per_slot > avail0) c.grid /= 2;
             c.nslots = (size_t)c.grid * T;
             max_slots = std::max(max_slots, c.nslots);
-            if (v) SWB_CUDA(cudaFuncSetAttribute(global_smem_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
-            else SWB_CUDA(cudaFuncSetAttribute(global_smem_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
+            // (the block limit, not c.smem: another thread's call may set it before the launch)
+            if (v) SWB_CUDA(cudaFuncSetAttribute(global_smem_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, blk_bytes));
+            else SWB_CUDA(cudaFuncSetAttribute(global_smem_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, blk_bytes));
         }
         z_bytes = std::max(z_bytes, (max_slots * per_slot + 1023) & ~(size_t)1023);
         if (z_bytes > avail0) return set_error(SWB_ERR_OOM, "global alignment scratch does not fit the memory budget");

@@ -1,9 +1,10 @@
-"""Calls of one context on several streams: a device entry returns while its
-pass runs, and the calls after it, on other streams or through host entries,
-use the same workspace.  Every call has to give the oracle's results.  Batches
-small enough for a warp per task and large enough for the bins to leave rows
-out, each next one larger (the workspace moves); the plain form; host batches
-of extensions and of global alignments in between."""
+"""Calls of one context on several streams, and of several contexts on several
+threads.  One context: a device entry returns while its pass runs, and the
+calls after it, on other streams or through host entries, use the same
+workspace.  Every call has to give the oracle's results.  Batches small enough
+for a warp per task and large enough for the bins to leave rows out, each next
+one larger (the workspace moves); the plain form; host batches of extensions
+and of global alignments in between."""
 import numpy as np
 import pytest
 
@@ -76,3 +77,40 @@ def test_passes_overlap_without_waiting_in_between(oracle_mod):
             assert np.array_equal(out.cpu().numpy().view(EXT_RESULT_DTYPE), exp[o])
     finally:
         eng.close()
+
+
+def test_contexts_on_several_threads(oracle_mod):
+    """Kernels whose shared memory a call sizes by its longest query, called from
+    two threads with different lengths (each its own context)."""
+    import threading
+    from swiftbwa_b200.alignment import Engine
+    sc = Scoring.default()
+    work = []
+    for k, qmax in enumerate((300, 3800)):
+        e = gen.ext_tasks(40 + k, 40, qmax=qmax)
+        g = gen.global_tasks(50 + k, 6000, qmax=40 if k else 250, retry=False)
+        exp, _ = oracle_mod.ext_batch(sc, e["bases"], e["tasks"], n_threads=8)
+        eres, _, _ = oracle_mod.global_batch(sc, g["bases"], g["tasks"], n_threads=8)
+        work.append((e, exp, g, eres))
+    errors = []
+
+    def loop(e, exp, g, eres):
+        eng = Engine(0)
+        try:
+            for turn in range(150):
+                if not np.array_equal(eng.ext_batch(sc, e["bases"], e["tasks"]), exp):
+                    raise AssertionError("extensions differ")
+                if turn % 5 == 0 and not np.array_equal(eng.global_batch(sc, g["bases"], g["tasks"])[0]["score"],
+                                                        eres["score"]):
+                    raise AssertionError("global alignments differ")
+        except Exception as x:   # noqa: BLE001 -- reported below, in the test's thread
+            errors.append(x)
+        finally:
+            eng.close()
+
+    th = [threading.Thread(target=loop, args=w) for w in work for _ in range(2)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not errors, errors[0]
