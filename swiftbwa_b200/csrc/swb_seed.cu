@@ -783,7 +783,7 @@ int swb_smem_batch(swb_ctx *ctx, const uint8_t *bases, size_t n_bases, const uin
         g.order = order;
     }
     {
-        ProfScope ps(ctx, st, "smem_search", kCntSeed);
+        ProfScope ps(ctx, st, compact ? "smem_search" : "smem_search_cp64", kCntSeed);
         if (compact) smem_kernel<uint32_t><<<(unsigned)blocks, kSeedT, 0, st>>>(g);
         else smem_kernel<int64_t><<<(unsigned)blocks, kSeedT, 0, st>>>(g);
     }

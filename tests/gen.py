@@ -157,10 +157,10 @@ def local_tasks(seed, n, qmax=260, tmax=800, ref_len=0):
     return dict(bases=np.concatenate(chunks), tasks=tasks)
 
 
-def ext_batch_binned(engine, sc, bases, tasks):
-    """Runs tasks through swb_ext_batch_device (HBM-resident inputs): always
-    the binned pass -- the host entry sends batches of up to 16384 tasks to
-    the one-launch form instead."""
+def ext_batch_device(engine, sc, bases, tasks):
+    """Runs tasks through swb_ext_batch_device (HBM-resident inputs): batches of
+    up to 4096 tasks run a warp per task (queries up to 4096), larger ones the
+    binned pass."""
     import torch
     from swiftbwa_b200.abi import EXT_RESULT_DTYPE
     d_b = torch.from_numpy(np.ascontiguousarray(bases)).to("cuda:0")
@@ -170,3 +170,23 @@ def ext_batch_binned(engine, sc, bases, tasks):
     engine.ext_batch_device(sc, d_b.data_ptr(), d_t.data_ptr(), len(tasks), d_o.data_ptr(), s.cuda_stream)
     s.synchronize()
     return d_o.cpu().numpy().view(EXT_RESULT_DTYPE)[: len(tasks)]
+
+
+def ext_batch_binned(engine, sc, bases, tasks):
+    """The binned pass over tasks, repeated past the size that runs a warp per
+    task -> (the first copy's results, the copies, {kernel: cells} of a second,
+    profiled run).  All copies, of both runs, have to agree."""
+    rep = 4096 // len(tasks) + 2
+    t = np.tile(tasks, rep)
+    got = ext_batch_device(engine, sc, bases, t)
+    engine.profile(True)
+    engine.profile_reset()
+    try:
+        every = ext_batch_device(engine, sc, bases, t)
+        prof = engine.profile_read()
+    finally:
+        engine.profile(False)
+    first = got[: len(tasks)]
+    assert np.array_equal(got, np.tile(first, rep)) and np.array_equal(every, got)
+    assert not any(k.startswith("ext_warps") for k in prof) and "ext_keys" in prof
+    return first, rep, {k: v[2] for k, v in prof.items() if k.startswith(("ext_u8_q", "ext_i16_q", "ext_big"))}

@@ -24,7 +24,7 @@ def test_extension_pass_without_room_for_rows_left_out():
         eng = Engine(0, mem_budget_bytes=budget + (1 << 20 if budget else 0))
         try:
             eng.upload_reference(ref.pac, ref.n)
-            got[budget] = gen.ext_batch_binned(eng, sc, wl.bases, wl.tasks)
+            got[budget] = gen.ext_batch_device(eng, sc, wl.bases, wl.tasks)
         except SWBError as e:
             got[budget] = e.status
         finally:

@@ -12,7 +12,8 @@ import numpy as np
 import pytest
 
 import gen
-from swiftbwa_b200.abi import EXT_TASK_DTYPE, SWB_Q_REVERSE, SWB_T_COMPLEMENT, SWB_T_REVERSE, Scoring
+from swiftbwa_b200.abi import (EXT_TASK_DTYPE, SWB_Q_REVERSE, SWB_T_COMPLEMENT, SWB_T_FROM_REF, SWB_T_REVERSE,
+                               Scoring)
 
 pytestmark = pytest.mark.gpu
 
@@ -81,10 +82,10 @@ def test_rows_left_out(oracle_mod, si, qmax, bins):
             eng.set_ext_bins(bins)
         for n, rep in ((1500, 1), (6000, 1), (6000, 17)):
             t, want = np.tile(tasks[:n], rep), np.tile(exp[:n], rep)
-            check(gen.ext_batch_binned(eng, sc, bases, t), want, t)
+            check(gen.ext_batch_device(eng, sc, bases, t), want, t)
             eng.profile(True)
             eng.profile_reset()
-            every = gen.ext_batch_binned(eng, sc, bases, t)
+            every = gen.ext_batch_device(eng, sc, bases, t)
             prof = eng.profile_read()
             eng.profile(False)
             check(every, want, t)
@@ -93,6 +94,46 @@ def test_rows_left_out(oracle_mod, si, qmax, bins):
             check(eng.ext_batch(sc, bases, t), want, t)
             if n == 6000:
                 assert eng.last_batch_stats()[1] == cells * rep
+    finally:
+        eng.close()
+
+
+def _on_reference(rng, bases, tasks):
+    """The tasks with their targets on a resident strand where they hold no N
+    (each behind 0-15 bases, so that spans begin anywhere in a word)."""
+    t, parts, at = tasks.copy(), [], 0
+    for k, x in enumerate(tasks):
+        span = bases[int(x["t_off"]):int(x["t_off"]) + int(x["tlen"])]
+        if x["tlen"] == 0 or (span > 3).any():
+            continue
+        gap = int(rng.integers(0, 16))
+        parts += [rng.integers(0, 4, gap).astype(np.uint8), span]
+        t["t_off"][k] = at + gap
+        t["flags"][k] |= SWB_T_FROM_REF
+        at += gap + len(span)
+    ref = np.concatenate(parts)
+    return t, gen.pack_ref(ref), len(ref)
+
+
+@pytest.mark.parametrize("si", [0, 2, 3])
+def test_rows_left_out_on_the_reference(oracle_mod, si):
+    """The same rules where targets are spans of the packed reference, either
+    strand and direction, in a pass that leaves rows out in the bins and in one
+    with a warp per task."""
+    from swiftbwa_b200.alignment import Engine
+    sc = Scoring.default(**SCORINGS[si])
+    bases, tasks = _tasks(1700 + si, 6000, 250)
+    tasks, pac, ref_bases = _on_reference(np.random.default_rng(si), bases, tasks)
+    assert ((tasks["flags"] & SWB_T_FROM_REF) != 0).sum() > 4000
+    exp, _ = oracle_mod.ext_batch(sc, bases, tasks, pac=pac, ref_bases=ref_bases, n_threads=8)
+    eng = Engine(0)
+    try:
+        eng.upload_reference(pac, ref_bases)
+        for n, rep in ((3000, 1), (6000, 17)):
+            t, want = np.tile(tasks[:n], rep), np.tile(exp[:n], rep)
+            got = gen.ext_batch_device(eng, sc, bases, t)
+            bad = np.nonzero(got != want)[0]
+            assert bad.size == 0, f"{len(t)}: {bad.size} mismatches, first {t[bad[:3]]}: {got[bad[:3]]} vs {want[bad[:3]]}"
     finally:
         eng.close()
 

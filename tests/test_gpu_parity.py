@@ -93,9 +93,15 @@ def test_ext_fuzz(engine, oracle_mod, si):
     assert bad.size == 0, f"{bad.size} mismatches, first {bad[:5]}: {got[bad[:3]]} vs {exp[bad[:3]]} tasks {d['tasks'][bad[:3]]}"
     ms, gcells = engine.last_batch_stats()
     assert gcells == cells
-    binned = gen.ext_batch_binned(engine, sc, d["bases"], d["tasks"])
+    small = gen.ext_batch_device(engine, sc, d["bases"], d["tasks"])
+    bad = _cmp_struct(small, exp, got.dtype.names)
+    assert bad.size == 0, f"a warp per task: {bad.size} mismatches, first {bad[:5]}"
+    binned, rep, kernels = gen.ext_batch_binned(engine, sc, d["bases"], d["tasks"])
     bad = _cmp_struct(binned, exp, got.dtype.names)
     assert bad.size == 0, f"binned: {bad.size} mismatches, first {bad[:5]}"
+    assert sum(kernels.values()) == cells * rep
+    assert any(k.startswith("ext_i16_q") and v for k, v in kernels.items())
+    assert any(k.startswith("ext_u8_q") and v for k, v in kernels.items())
 
 
 @pytest.mark.parametrize("si", [0, 1, 3])
@@ -107,18 +113,19 @@ def test_ext_ring_rows(engine, oracle_mod, si):
     sc = Scoring.default(**SCORINGS[si])
     d = gen.ext_tasks(4242 + si, 1500, qmax=2500, ref_len=20000)
     engine.upload_reference(d["pac"], d["ref_bases"])
-    engine.profile(True)
-    engine.profile_reset()
-    try:
-        got = gen.ext_batch_binned(engine, sc, d["bases"], d["tasks"])
-        prof = engine.profile_read()
-    finally:
-        engine.profile(False)
+    got, rep, kernels = gen.ext_batch_binned(engine, sc, d["bases"], d["tasks"])
     exp, cells = oracle_mod.ext_batch(sc, d["bases"], d["tasks"], pac=d["pac"], ref_bases=d["ref_bases"],
                                       n_threads=8)
     bad = _cmp_struct(got, exp, got.dtype.names)
     assert bad.size == 0, f"{bad.size} mismatches, first {bad[:5]}: {got[bad[:3]]} vs {exp[bad[:3]]} tasks {d['tasks'][bad[:3]]}"
-    assert sum(v[2] for k, v in prof.items() if k.startswith("ext_")) == cells
+    assert sum(kernels.values()) == cells * rep
+    # Queries that no class holds: cells of a shared-memory bin are a ring's.
+    long = d["tasks"][d["tasks"]["qlen"] > 256]
+    got, rep, kernels = gen.ext_batch_binned(engine, sc, d["bases"], long)
+    bad = _cmp_struct(got, exp[d["tasks"]["qlen"] > 256], got.dtype.names)
+    assert bad.size == 0, f"long queries: {bad.size} mismatches"
+    ring = sum(v for k, v in kernels.items() if not k.startswith("ext_big"))
+    assert 0 < ring < sum(kernels.values())
 
 
 def test_ext_host_entry_small_batch_threshold(engine, oracle_mod):
@@ -159,9 +166,12 @@ def test_ext_length_classes(engine, oracle_mod, bins):
     try:
         engine.set_ext_bins(bins)
         assert engine.ext_bins() == bins
-        got = gen.ext_batch_binned(engine, sc, d["bases"], d["tasks"])
+        got, rep, kernels = gen.ext_batch_binned(engine, sc, d["bases"], d["tasks"])
         bad = _cmp_struct(got, exp, got.dtype.names)
         assert bad.size == 0, f"{bins}: {bad.size} mismatches, first {bad[:5]}"
+        assert sum(kernels.values()) == cells * rep
+        used = {int(k.rsplit("_q", 1)[1]) for k, v in kernels.items() if "_q" in k and v}
+        assert used == set(bins), f"classes with cells: {used}"
     finally:
         engine.set_ext_bins(default)
 
@@ -204,15 +214,17 @@ def test_global_fuzz(engine, oracle_mod, si, qmax):
     within the shared-memory kernels."""
     sc = Scoring.default(**(BIG_PENALTIES if si == "big" else SCORINGS[si]))
     d = gen.global_tasks(2000 + (7 if si == "big" else si) + qmax, 1500, qmax=qmax)
-    res, cig = engine.global_batch(sc, d["bases"], d["tasks"])
     eres, ecig, _ = oracle_mod.global_batch(sc, d["bases"], d["tasks"], n_threads=8)
-    for k in range(len(res)):
-        assert res["score"][k] == eres["score"][k], k
-        assert res["n_cigar"][k] == eres["n_cigar"][k], k
-        assert res["w_used"][k] == eres["w_used"][k] and res["attempts"][k] == eres["attempts"][k], k
-        o, n = int(res["cigar_off"][k]), int(res["n_cigar"][k])
-        eo = int(eres["cigar_off"][k])
-        assert np.array_equal(cig[o:o + n], ecig[eo:eo + n]), k
+    m = len(eres)
+    for rep in (1, 4):   # a warp per int16-row alignment, and a thread each
+        res, cig = engine.global_batch(sc, d["bases"], np.tile(d["tasks"], rep))
+        for f in ("score", "n_cigar", "w_used", "attempts"):
+            bad = np.nonzero(res[f] != np.tile(eres[f], rep))[0]
+            assert bad.size == 0, f"{rep} copies: {f} differs for {bad.size}, first {bad[:5]}"
+        for k in range(len(res)):
+            o, n = int(res["cigar_off"][k]), int(res["n_cigar"][k])
+            eo = int(eres["cigar_off"][k % m])
+            assert np.array_equal(cig[o:o + n], ecig[eo:eo + n]), (rep, k)
 
 
 @pytest.mark.parametrize("si", [0, 3, 4, 5])

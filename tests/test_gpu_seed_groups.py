@@ -56,9 +56,12 @@ def test_groups_equal_oracle(oracle_mod, wide, n, lmax):
     eng = Engine(0)
     try:
         eng.upload_bwt(cp, idx.count, idx.length, idx.sentinel)
+        eng.profile(True)
         got, gn, goff = eng.smem_batch(bases, off, lens, 15, cap_per_read=cap, split_len=28)
+        ran = [k for k in eng.profile_read() if k.startswith("smem_search")]
     finally:
         eng.close()
+    assert ran == (["smem_search_cp64"] if wide else ["smem_search"])
     assert np.array_equal(gn, en)
     for r in range(n):
         assert np.array_equal(got[goff[r]:goff[r] + gn[r]], exp[r * cap:r * cap + en[r]]), f"read {r}"
