@@ -281,7 +281,9 @@ int swb_get_ext_bins(swb_ctx *ctx, int32_t *qmax, int cap, int *n);
  * quantiles of the batch's row lengths and estimated cells) on the given
  * sample batch (host arrays, as swb_ext_batch; best of two runs after a
  * warm-up each) and keeps the fastest in the context, the defaults unless
- * another set is more than 2 % faster.  Writes the chosen classes
+ * another set is more than 2 % faster.  The timed pass is that of
+ * swb_ext_batch_device; swb_ext_batch, the chains and the server use the same
+ * classes but also compute the last rows (see swb_profile).  Writes the chosen classes
  * (qmax_out[0..cap), *n_out), the chosen set's and the defaults' time on
  * the sample (ms; may be NULL). */
 int swb_tune_ext_bins(swb_ctx *ctx, const swb_scoring *sc, const uint8_t *bases, size_t n_bases,
