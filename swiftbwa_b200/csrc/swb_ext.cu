@@ -14,8 +14,8 @@
 //     everything else (rows above the last bound, larger scores, gap costs
 //     beyond a 16-bit lane) goes to the int32 bin.
 //     The bounds are static, so no row ever saturates and nothing is re-run.
-//     A CUB radix sort orders the tasks by (bin, longest query, longest
-//     target).
+//     A CUB radix sort orders the tasks by (bin, widest band, most rows left,
+//     longest row): ext_keys_kernel.
 //   * Every shared-memory bin is one launch of a persistent grid of one-warp
 //     blocks; lane 0 claims the next 32 sorted tasks of the bin from a device
 //     counter, so long tasks start first and no block holds a bin up.  The

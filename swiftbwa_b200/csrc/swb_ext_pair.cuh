@@ -57,8 +57,8 @@
 // left) below gScore and not above maxScore, for every nonzero word -- the
 // rows left change nothing (a path only loses by gaps, a zero cell starts
 // none, z-drop and an empty row only stop earlier).  ALL = true computes them,
-// for callers that report the reference's cell count; the skipped first rows'
-// cells are counted from the band either way.
+// for callers that report the reference's cell count; it also counts the first
+// rows' cells from their bands.  With ALL = false neither is counted.
 #pragma once
 
 #include <type_traits>

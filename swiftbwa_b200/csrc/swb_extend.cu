@@ -16,7 +16,8 @@
 //                  then feed each result back: the chain either emits its
 //                  next task (retry, right side, next seed) or finishes.
 //
-// The host only reads one count per round.  Regions are written in place
+// The host reads one count per round, and the bin sizes of a round that runs
+// the bins.  Regions are written in place
 // (chain c's at out[seed_off ...]) and copied back once at the end.
 #include <algorithm>
 #include <thread>
@@ -502,8 +503,11 @@ extern "C" int swb_extend_chains(swb_ctx *ctx, const swb_scoring *sc, const uint
         SWB_CUDA(cudaStreamSynchronize(st));
         if (n == 0) break;
         // A round that runs the bins has its bin sizes read back (no hint), so that
-        // the ones without tasks, most of them for short reads, are not launched (200k
-        // chains of 150 bp reads, two rounds: 5.77 -> 5.38 and 5.78 -> 4.72 ms in two runs).
+        // the ones without tasks, most of them for short reads, are not launched.
+        // Without / with, medians of 40 calls in three runs: 150 bp reads, 10k chains
+        // 1.13-1.15 / 1.13-1.24 ms, 20k 1.47-1.50 / 1.42-1.45, 50k 1.90-2.27 /
+        // 1.68-1.71, 200k 3.80-4.48 / 3.48-3.97; 250 bp, 10k 2.06-2.13 / 1.90-1.91,
+        // 50k 3.42-3.72 / 2.63-2.65, 200k 6.80-7.44 / 5.89-6.85.
         const int hint = n > kExtWarpsMaxTasks ? -1 : max_read;
         if ((rc = launch_ext(ctx, dsc, (const uint8_t *)ctx->d_bases.p, d_batch, n, d_res, ctx->d_counters, st, hint, 0,
                              nullptr, true, true)))

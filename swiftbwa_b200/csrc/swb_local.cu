@@ -76,7 +76,9 @@ struct PassOut {
 // and three full-rate instructions.  Bound by the ALU pipe and issue.  Against
 // 16 threads a task with one lane each and 32-bit values (two tasks a warp,
 // both passes in one launch per stripe count), 50k pairs of 150 x 700 went
-// from 9.29 to 3.30 ms (880 -> 2480 GCUPS).
+// from 9.29 to 3.30 ms (forward launch 2.29 ms, issue 71 %).  Part of that is the
+// reverse pass stopping early (rev_cap); its columns left out count as cells all
+// the same.
 //
 // WRAP: H + profile may pass 255 while H <= 250, so the reference's UInt8
 // wrap is applied; else it cannot happen (H > 250 ends the pass, :247).

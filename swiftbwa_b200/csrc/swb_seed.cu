@@ -367,7 +367,7 @@ struct Walker {
 // call at 12.8 ms; eight threads need 240 and 1,150.  Kernel time on a 100 Mbp
 // index, 100k reads 12.8 -> 2.74 ms, 1M reads 39.9 -> 23.8 ms (four threads a
 // read: 3.45 ms per 100k, sixteen: 3.77; ten blocks per SM 3.13, six 2.90).
-// Bound by instruction issue (about 320 a round, 70 % of the issue slots).
+// Bound by instruction issue (about 320 a round, 77 % of the issue slots).
 // Control flow is uniform over the warp outside of short branches without
 // synchronisation, so that its groups stay together (with a transition loop
 // per group they ran the extension apart, 13.8 threads an instruction, 6.2 ms).
