@@ -253,11 +253,12 @@ extern "C" int swb_cigar_batch(swb_ctx *ctx, const swb_scoring *sc, const uint8_
                 const int32_t deficit = t.qlen * sc->a - t.true_score;
                 fast[i] = t.qlen == t.rlen && t.qlen > 0 && deficit < min_indel;
                 if (fast[i]) continue;
-                if (r.band_bad == SIZE_MAX && t.qlen > 0 && t.rlen > 0 && std::max(band_of(t), std::abs(t.qlen - t.rlen)) < 1)
+                const int32_t band = band_of(t);
+                if (r.band_bad == SIZE_MAX && t.qlen > 0 && t.rlen > 0 && std::max(band, std::abs(t.qlen - t.rlen)) < 1)
                     r.band_bad = i;
                 ++r.nd;
                 r.raw += (size_t)t.qlen + (size_t)t.rlen;
-                r.shape.add(t.qlen, t.rlen, band_of(t), cost16);
+                r.shape.add(t.qlen, t.rlen, band, cost16);
             }
         });
     }

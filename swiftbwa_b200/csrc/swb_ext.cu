@@ -56,8 +56,7 @@ namespace {
 // int32 rows (one warp per extension, or global scratch above kWarpMaxQ).
 constexpr int kFastT = 32;                // threads per block in the shared-memory kernels
 // Per pass: bin bounds (up to 32 words), the int32 bin's longest query at
-// byte 256, a zero at byte 264 (passes without rows left out), the bins' claim
-// counters from byte 320.
+// byte 256, the bins' claim counters from byte 320.
 constexpr size_t kMiscBytes = 512;
 constexpr int kBigT = 64;
 constexpr size_t kSmemPerSm = 227 * 1024;
@@ -155,8 +154,10 @@ __global__ void bin_bounds_kernel(const uint32_t *__restrict__ sorted_keys, size
 
 // qcap: the bin's class bound.  (An instance per bound, with it as a constant,
 // ran 1-4 % slower than this one: 31 instances' code for an inner loop that
-// does not use the bound.)
-template <int T, bool U8, bool ALL, bool AHEAD>
+// does not use the bound.)  SKIP: the pass has rows left out (a.skip); without,
+// the loads run ahead (an instance of its own costs the others nothing: a NULL
+// check or a masked index took 0.3-1.2 % of 2M reads).
+template <int T, bool U8, bool ALL, bool AHEAD, bool SKIP>
 __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qcap) {
     extern __shared__ uint32_t sm[];
     // Rows: (qcap + 1) words of 2 (int8 scores) or 4 bytes (int16), then
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qca
         if (pos < hi) {
             swb_ext_result r;
             const bool sym = a.sc.o_del + a.sc.e_del == a.sc.o_ins + a.sc.e_ins;
-            const int skip = a.skip[ti & a.skip_mask];
+            const int skip = SKIP ? a.skip[ti] : 0;
             auto run = [&](auto symc, auto ringc) {
                 constexpr bool kSym = decltype(symc)::value, kRing = decltype(ringc)::value;
                 if constexpr (U8) ext_pair_one<T, kSym, false, kRing, ALL, AHEAD>(a, tk, skip, he16, qc, r, cells);
@@ -398,28 +399,30 @@ const char *bin_name(bool u8, int qcap) {
 
 using FastKernel = void (*)(ExtArgs, int, int);
 
-template <bool U8>
-FastKernel fast_kernel_of(bool all, bool ahead) {
-    if (all) return ahead ? ext_fast_kernel<kFastT, U8, true, true> : ext_fast_kernel<kFastT, U8, true, false>;
-    return ahead ? ext_fast_kernel<kFastT, U8, false, true> : ext_fast_kernel<kFastT, U8, false, false>;
+// (Without rows left out, ahead is always true.)
+template <bool U8, bool ALL>
+FastKernel fast_kernel_of(bool ahead, bool skip) {
+    if (!skip) return ext_fast_kernel<kFastT, U8, ALL, true, false>;
+    return ahead ? ext_fast_kernel<kFastT, U8, ALL, true, true> : ext_fast_kernel<kFastT, U8, ALL, false, true>;
 }
-FastKernel fast_kernel(bool u8, bool all, bool ahead) {
-    return u8 ? fast_kernel_of<true>(all, ahead) : fast_kernel_of<false>(all, ahead);
+FastKernel fast_kernel(bool u8, bool all, bool ahead, bool skip) {
+    return u8 ? (all ? fast_kernel_of<true, true>(ahead, skip) : fast_kernel_of<true, false>(ahead, skip))
+              : (all ? fast_kernel_of<false, true>(ahead, skip) : fast_kernel_of<false, false>(ahead, skip));
 }
 
 // Resident one-warp blocks per SM of the shared-memory kernel for a class bound.
-int fast_occupancy(bool u8, bool all, bool ahead, int qcap) {
-    static int cache[8][kExtSmemMaxQ + 1];
+int fast_occupancy(bool u8, bool all, bool ahead, bool skip, int qcap) {
+    static int cache[16][kExtSmemMaxQ + 1];
     static std::once_flag once;
     std::call_once(once, [] {
         for (auto &row : cache)
             for (int &v : row) v = -1;
     });
-    int &occ = cache[(u8 ? 1 : 0) + (all ? 2 : 0) + (ahead ? 4 : 0)][qcap];
+    int &occ = cache[(u8 ? 1 : 0) + (all ? 2 : 0) + (ahead ? 4 : 0) + (skip ? 8 : 0)][qcap];
     if (occ < 0) {
         int o = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8, all, ahead), kFastT, fast_smem_bytes(qcap, u8)) !=
-            cudaSuccess)
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fast_kernel(u8, all, ahead, skip), kFastT,
+                                                          fast_smem_bytes(qcap, u8)) != cudaSuccess)
             return -1;
         occ = o < 1 ? 1 : o;
     }
@@ -434,22 +437,22 @@ int fast_occupancy(bool u8, bool all, bool ahead, int qcap) {
 // 150 bp reads: 16k 532 / 533, 64k 684 / 710, 1M 2232 / 2998).
 bool leaves_first_rows(const swb_ctx *ctx, size_t n) { return n > (size_t)ctx->sm_count * 20 * kFastT; }
 
-// n: the pass's tasks; in_bin: at least the bin's.
-int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, size_t in_bin,
-                cudaStream_t s) {
+// in_bin: at least the bin's tasks.
+int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t in_bin, cudaStream_t s) {
     // Loads a step ahead where latency counts: rows that leave room for fewer
-    // than kAheadBlocks blocks per SM, and passes that do not fill the SMs.
+    // than kAheadBlocks blocks per SM, and passes that do not fill the SMs, which
+    // have no rows left out (leaves_first_rows; nor have those without room for them).
     // Without / with in every bin / by this rule: 131k uneven tasks 1431 / 1266 /
     // 1249 us, 5M 28.9 / 26.9 / 26.8 ms; 2M tasks of 150 bp reads 3772 / 3908 /
     // 3779 us.
-    const bool ahead = n <= (size_t)ctx->sm_count * 20 * kFastT || fast_smem_bytes(qcap, u8) * kAheadBlocks > kSmemPerSm;
-    const int occ = fast_occupancy(u8, all, ahead, qcap);
+    const bool skip = a.skip != nullptr, ahead = !skip || fast_smem_bytes(qcap, u8) * kAheadBlocks > kSmemPerSm;
+    const int occ = fast_occupancy(u8, all, ahead, skip, qcap);
     if (occ < 0) return check_cuda(cudaGetLastError(), "occupancy query");
     const size_t grid = std::min<size_t>((in_bin + kFastT - 1) / kFastT, (size_t)ctx->sm_count * occ);
     if (grid == 0) return SWB_OK;
     const size_t smem = fast_smem_bytes(qcap, u8);
     ProfScope ps(ctx, s, ctx->prof_on ? bin_name(u8, qcap) : nullptr, kCntExtBin0 + bin);
-    fast_kernel(u8, all, ahead)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
+    fast_kernel(u8, all, ahead, skip)<<<(unsigned)grid, kFastT, smem, s>>>(a, bin, qcap);
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
     return SWB_OK;
@@ -553,7 +556,6 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     char *misc = (char *)ctx->d_misc.p + slot * kMiscBytes;
     uint32_t *bin_start = (uint32_t *)misc;                   // nbins + 1 words
     int *big_max_q = (int *)(misc + 256);
-    const uint16_t *no_skip = (const uint16_t *)(misc + 264);   // a zero
     uint32_t *claim = (uint32_t *)(misc + 320);               // nbins claim counters
     SWB_CUDA(cudaMemsetAsync(misc + 256, 0, kMiscBytes - 256, s));   // big_max_q and the counters
     const unsigned tb = 256;
@@ -567,10 +569,9 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     }
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
-    size_t tmp_bytes = 0;
-    SWB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, idx, idx2, (int)n, 0, 32, s));
     {
         ProfScope ps(ctx, s, "cub_radix_sort", -1);
+        size_t tmp_bytes = ctx->d_sort_tmp.cap;   // (at least what ext_workspace found the sort to need)
         SWB_CUDA(cub::DeviceRadixSort::SortPairs(ctx->d_sort_tmp.p, tmp_bytes, keys, keys2, idx, idx2,
                                                  (int)n, 0, 32, s));
     }
@@ -613,8 +614,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
 
     // Fork: every bin runs on its own stream after the sort, then joins back
     // (into the pipeline's join stream for pipelined passes).
-    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, d_cells, claim, ring_above, skip ? skip : no_skip,
-              skip ? 0xFFFFFFFFu : 0u};
+    ExtArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, d_cells, claim, ring_above, skip};
     const cudaStream_t js = pipe ? pipe->join : s;
     ProfScope pass(ctx, s, pipe ? nullptr : "ext_pass", -1);   // fork to join, on the launching stream
     SWB_CUDA(cudaEventRecord(ctx->fork_ev, s));
@@ -628,7 +628,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         SWB_CUDA(cudaStreamWaitEvent(sb, ctx->fork_ev, 0));
         if (b < big) {
             const size_t in_bin = sized ? shape[b + 1] - shape[b] : n;
-            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], n, in_bin, sb))) return rc;
+            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], in_bin, sb))) return rc;
         } else {
             ProfScope ps(ctx, sb, "ext_big_i32", kCntExtBin0 + big);
             ext_warp_kernel<<<(unsigned)wblocks, wwarps * 32, wwarps * wstride, sb>>>(a, big, wq);

@@ -20,8 +20,7 @@ struct ExtArgs {
     unsigned long long *cells;
     uint32_t *claim = nullptr;  // per-bin claim counters (zeroed per pass)
     int ring_above = 0x7FFFFFFF;   // queries longer than this keep their band as a ring (ext_row_len)
-    const uint16_t *skip = nullptr;   // per task, the first rows it leaves out (ext_skip_rows)
-    uint32_t skip_mask = 0;           // of the task's index into skip (0: one zero for all)
+    const uint16_t *skip = nullptr;   // per task, the first rows it leaves out (ext_skip_rows); NULL: none
 };
 
 // ---------------------------------------------------------------- row stores
