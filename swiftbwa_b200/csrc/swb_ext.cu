@@ -109,7 +109,7 @@ __device__ __forceinline__ int ext_bin(const swb_ext_task &t, const DevScoring &
 // to the target's end, or with all = 0 about the query's length, where most
 // tasks stop.
 __global__ void ext_keys_kernel(const swb_ext_task *__restrict__ tasks, size_t n, DevScoring sc, int pair_ok,
-                                uint32_t warp_cells, ExtBins bins, int ring_above, int all,
+                                uint32_t warp_cells, ExtBins bins, int ring_above, int all, int skip_rows,
                                 const uint8_t *__restrict__ bases, const uint8_t *__restrict__ pac,
                                 uint32_t *__restrict__ keys, uint32_t *__restrict__ idx, uint16_t *__restrict__ skip,
                                 int *__restrict__ big_max_q) {
@@ -119,7 +119,7 @@ __global__ void ext_keys_kernel(const swb_ext_task *__restrict__ tasks, size_t n
     int len = task_row_len(t, sc, ring_above), s = 0;
     int b = ext_bin(t, sc, pair_ok != 0, warp_cells, bins, len);
     const bool pair = b < 2 * bins.n && t.qlen > 0 && t.tlen > 0;
-    if (pair && skip && len == t.qlen) {
+    if (pair && skip && skip_rows && len == t.qlen) {
         s = ext_skip_rows(t, sc, bases, pac);
         if (s > 0) {   // the columns left: maybe a smaller class
             len -= ext_start_col(sc, ext_band_w(t.qlen, t.w, t.end_bonus, sc), t.h0, s);
@@ -154,9 +154,10 @@ __global__ void bin_bounds_kernel(const uint32_t *__restrict__ sorted_keys, size
 
 // qcap: the bin's class bound.  (An instance per bound, with it as a constant,
 // ran 1-4 % slower than this one: 31 instances' code for an inner loop that
-// does not use the bound.)  SKIP: the pass has rows left out (a.skip); without,
-// the loads run ahead (an instance of its own costs the others nothing: a NULL
-// check or a masked index took 0.3-1.2 % of 2M reads).
+// does not use the bound.)  SKIP: the pass has the array of rows left out; without
+// it, the loads run ahead.  (A NULL check or a masked index in one instance for
+// both took 0.3-1.2 % of 2M reads.  Small passes, whose array holds zeros, keep
+// SKIP: without it 5k-94k uneven tasks of up to 400 bases run 7-9 % longer.)
 template <int T, bool U8, bool ALL, bool AHEAD, bool SKIP>
 __global__ void __launch_bounds__(T) ext_fast_kernel(ExtArgs a, int bin, int qcap) {
     extern __shared__ uint32_t sm[];
@@ -399,7 +400,7 @@ const char *bin_name(bool u8, int qcap) {
 
 using FastKernel = void (*)(ExtArgs, int, int);
 
-// (Without rows left out, ahead is always true.)
+// (Without the array, always ahead.)
 template <bool U8, bool ALL>
 FastKernel fast_kernel_of(bool ahead, bool skip) {
     if (!skip) return ext_fast_kernel<kFastT, U8, ALL, true, false>;
@@ -431,21 +432,22 @@ int fast_occupancy(bool u8, bool all, bool ahead, bool skip, int qcap) {
 
 // The rows before the first mismatch are left out in passes of more tasks
 // than the GPU holds lanes of these kernels (about 20 one-warp blocks per
-// SM).  A smaller pass lasts as long as its longest task, and lanes that
+// SM) that have room for the array.  A smaller pass lasts as long as its longest task, and lanes that
 // start at different rows take longer over each (uneven tasks, rows left out
 // / kept: 8k 1455 / 1242 us, 64k 1436 / 1330, 256k 2169 / 2310, 1M 6679 / 7731;
 // 150 bp reads: 16k 532 / 533, 64k 684 / 710, 1M 2232 / 2998).
 bool leaves_first_rows(const swb_ctx *ctx, size_t n) { return n > (size_t)ctx->sm_count * 20 * kFastT; }
 
-// in_bin: at least the bin's tasks.
-int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t in_bin, cudaStream_t s) {
+// n: the pass's tasks; in_bin: at least the bin's.
+int launch_fast(swb_ctx *ctx, const ExtArgs &a, int bin, bool u8, bool all, int qcap, size_t n, size_t in_bin,
+                cudaStream_t s) {
     // Loads a step ahead where latency counts: rows that leave room for fewer
-    // than kAheadBlocks blocks per SM, and passes that do not fill the SMs, which
-    // have no rows left out (leaves_first_rows; nor have those without room for them).
+    // than kAheadBlocks blocks per SM, and passes that do not fill the SMs.
     // Without / with in every bin / by this rule: 131k uneven tasks 1431 / 1266 /
     // 1249 us, 5M 28.9 / 26.9 / 26.8 ms; 2M tasks of 150 bp reads 3772 / 3908 /
     // 3779 us.
-    const bool skip = a.skip != nullptr, ahead = !skip || fast_smem_bytes(qcap, u8) * kAheadBlocks > kSmemPerSm;
+    const bool skip = a.skip != nullptr;
+    const bool ahead = !skip || !leaves_first_rows(ctx, n) || fast_smem_bytes(qcap, u8) * kAheadBlocks > kSmemPerSm;
     const int occ = fast_occupancy(u8, all, ahead, skip, qcap);
     if (occ < 0) return check_cuda(cudaGetLastError(), "occupancy query");
     const size_t grid = std::min<size_t>((in_bin + kFastT - 1) / kFastT, (size_t)ctx->sm_count * occ);
@@ -472,7 +474,7 @@ static int ext_workspace(swb_ctx *ctx, size_t cap, int sets) {
         (rc = ensure_dev(ctx, ctx->d_idx, cap * 4)) || (rc = ensure_dev(ctx, ctx->d_misc, sets * kMiscBytes)) ||
         (rc = ensure_dev(ctx, ctx->d_sort_tmp, tmp_bytes)))
         return rc;
-    if (leaves_first_rows(ctx, cap) && ensure_dev(ctx, ctx->d_idx2, sets * cap * 6) == SWB_OK) return SWB_OK;
+    if (ensure_dev(ctx, ctx->d_idx2, sets * cap * 6) == SWB_OK) return SWB_OK;
     return ensure_dev(ctx, ctx->d_idx2, sets * cap * 4);
 }
 
@@ -550,7 +552,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
     uint32_t *keys = (uint32_t *)ctx->d_keys.p, *keys2 = (uint32_t *)ctx->d_keys2.p;
     uint32_t *idx = (uint32_t *)ctx->d_idx.p, *idx2 = (uint32_t *)ctx->d_idx2.p + (size_t)slot * set;
     // The rows each task leaves out, behind the sets' orders (ext_workspace).
-    uint16_t *skip = leaves_first_rows(ctx, n) && ctx->d_idx2.cap >= orders * 6
+    uint16_t *skip = ctx->d_idx2.cap >= orders * 6
                          ? (uint16_t *)((uint32_t *)ctx->d_idx2.p + orders) + (size_t)slot * set
                          : nullptr;
     char *misc = (char *)ctx->d_misc.p + slot * kMiscBytes;
@@ -564,8 +566,8 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         // Two target rows per pass on 16-bit lanes: the gap costs must fit a lane.
         const int pair_ok = sc.o_del + sc.e_del <= 32767 && sc.o_ins + sc.e_ins <= 32767;
         ext_keys_kernel<<<(unsigned)((n + tb - 1) / tb), tb, 0, s>>>(d_tasks, n, sc, pair_ok, warp_cells, bins,
-                                                                       ring_above, all, d_bases, ctx->d_pac,
-                                                                       keys, idx, skip, big_max_q);
+                                                                       ring_above, all, leaves_first_rows(ctx, n), d_bases,
+                                                                       ctx->d_pac, keys, idx, skip, big_max_q);
     }
     ctx->launches++;
     SWB_CUDA(cudaGetLastError());
@@ -628,7 +630,7 @@ int launch_ext(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases,
         SWB_CUDA(cudaStreamWaitEvent(sb, ctx->fork_ev, 0));
         if (b < big) {
             const size_t in_bin = sized ? shape[b + 1] - shape[b] : n;
-            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], in_bin, sb))) return rc;
+            if ((rc = launch_fast(ctx, a, b, b < bins.n, all, bins.q[b % bins.n], n, in_bin, sb))) return rc;
         } else {
             ProfScope ps(ctx, sb, "ext_big_i32", kCntExtBin0 + big);
             ext_warp_kernel<<<(unsigned)wblocks, wwarps * 32, wwarps * wstride, sb>>>(a, big, wq);
