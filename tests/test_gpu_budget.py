@@ -111,3 +111,28 @@ def test_global_batch_whose_warps_would_take_the_long_queries_scratch(oracle_mod
     for k in range(len(tasks)):
         o, n, eo = int(res["cigar_off"][k]), int(res["n_cigar"][k]), int(eres["cigar_off"][k])
         assert np.array_equal(cig[o:o + n], ecig[eo:eo + n]), k
+
+
+def test_host_batch_without_room_for_rows_left_out(oracle_mod):
+    """The pipelined host entry (several chunks, two orders) with the least budget
+    that it is not refused."""
+    from swiftbwa_b200 import workloads as W
+    from swiftbwa_b200.alignment import Engine, SWBError
+    ref = W.reference(W.SEED_BASE + 67, 2_000_000)
+    wl = W.uneven(ref, 68, 600_000, qmin=30, qmax=60, wmin=5, wmax=20)
+    sc = Scoring.default()
+
+    def call(budget):
+        eng = Engine(0, mem_budget_bytes=budget)
+        try:
+            eng.upload_reference(ref.pac, ref.n)
+            return eng.ext_batch(sc, wl.bases, wl.tasks), eng.last_batch_stats()[1]
+        except SWBError as e:
+            assert e.status == abi.SWB_ERR_OOM
+            return None
+        finally:
+            eng.close()
+
+    got, cells = call(_least_budget(call, 1 << 20, 1 << 28))
+    exp, want = oracle_mod.ext_batch(sc, wl.bases, wl.tasks, pac=ref.pac, ref_bases=ref.n, n_threads=8)
+    assert np.array_equal(got, exp) and cells == want
