@@ -100,7 +100,7 @@ struct PassOut {
 // to the striped shortcuts), so the reverse maximum is the forward score.
 // (WRAP: the arithmetic may lose alignments, so only a*qLen bounds it.)
 __device__ __forceinline__ int rev_cap(const DevScoring &sc, bool wrap, int qLen, int fwd_score) {
-    const int gOEE = ((sc.o_ins + sc.e_ins) & 0xFF) + (sc.e_ins & 0xFF);   // the bytes that striped_pass uses
+    const int gOEE = sc.o_ins + 2 * sc.e_ins;
     return !wrap && fwd_score >= sc.a * (qLen - 1) - gOEE ? fwd_score : sc.a * qLen;
 }
 
@@ -576,8 +576,12 @@ int launch_local(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases, con
 
     // Forward pass; the reverse keys go to `keys` (0 = nothing to do), then
     // the sort by them takes the forward order to the reverse one in `idx`.
+    // The striped passes take the gap costs as their bytes hold them (mate rescue
+    // allows more than 255), the scalar kernel as they are.
     LocalArgs a{sc, d_bases, ctx->d_pac, d_tasks, d_out, idx2, bin_start, fallback, fallback_n, d_cells, claim,
                 keys, peaks, peak_stride};
+    a.sc.e_ins = sc.e_ins & 0xFF;
+    a.sc.o_ins = ((sc.o_ins + sc.e_ins) & 0xFF) - a.sc.e_ins;
     SWB_CUDA(cudaMemsetAsync(keys, 0, n * 4, st));
     for (int h = ranges - 1; h >= 0; --h) {
         ProfScope ps(ctx, st, "local_striped_fwd", kCntLocalStriped);
@@ -600,6 +604,7 @@ int launch_local(swb_ctx *ctx, const DevScoring &sc, const uint8_t *d_bases, con
         SWB_CUDA(cudaGetLastError());
     }
     {
+        a.sc = sc;
         ProfScope ps(ctx, st, "local_scalar_i32", kCntLocalScalar);
         local_scalar_kernel<<<(unsigned)(nsl / kST), kST, 0, st>>>(a, hbuf, ebuf, pbuf, nsl);
     }
