@@ -441,7 +441,8 @@ typedef struct swb_smem {
  * bwtCountsBuffer / bwtSentinelBuffer (MetalSWEngine.swift:88-120).  The
  * checkpoints are kept as 32-byte blocks when length is below 2^32 - 1 and
  * every position but the sentinel's is in exactly one bitstring, else as
- * given; the results are the same. */
+ * given; the results are the same.  An index whose given form does not fit the
+ * memory budget is refused (SWB_ERR_OOM) and the one uploaded before stays. */
 int swb_upload_bwt(swb_ctx *ctx, const swb_bwt_checkpoint *cp, uint64_t n_cp, const int64_t count[5],
                    int64_t length, int64_t sentinel);
 
